@@ -116,6 +116,26 @@ __host__ __device__ constexpr int fixed_plane_stride(int d, int W) {
   return d == 3 ? (fixed_t_mid(d, W) + W - 1) * fixed_row_stride(d, W) : fixed_row_stride(d, W);
 }
 
+// The FP64 form's tiles (kernels_fix.cuh): 8 x 16 inner window starts in 3D for every W,
+// since tiles too large for shared memory go through it in slabs of planes.
+__host__ __device__ constexpr int fix_t_last(int d) { return d == 3 ? 16 : (d == 2 ? 64 : 1); }
+__host__ __device__ constexpr int fix_t_mid(int d) { return d == 3 ? 8 : 1; }
+__host__ __device__ constexpr int fix_row_stride(int d, int W) {
+  return d == 1 ? 0 : conflict_free_stride(fix_t_last(d) + W - 1, W);
+}
+__host__ __device__ constexpr int fix_plane_stride(int d, int W) {
+  return d == 3 ? (fix_t_mid(d) + W - 1) * fix_row_stride(d, W) : fix_row_stride(d, W);
+}
+
+// Constants of the FP64 form's fixed-point gridding (kernels_fix.cuh), one set per plan.
+struct FixPar {
+  uint64_t c60[kMaxDim];  // Gaussian: log2(e) / b_t in units of 2^-60 and of 2^-57
+  int64_t c57[kMaxDim];
+  double es_b2[kMaxDim];  // ES: beta_t log2(e)
+  int vbits;              // interpolation: bits of the scaled tile
+  int planes;             // d = 3: tile planes per slab (set per launch)
+};
+
 // Tiling of the oversampled grid used by the gridding kernels.
 struct Tiling {
   int T[kMaxDim];        // tile extent per dim (power of two, <= n_t)

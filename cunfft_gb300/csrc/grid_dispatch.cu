@@ -1,5 +1,7 @@
 // grid_dispatch.cu -- selects the gridding kernel instance for the plan's tap count.
-#include "kernels_grid.cuh"
+#include <math.h>
+
+#include "kernels_fix.cuh"
 
 namespace cg {
 
@@ -10,10 +12,44 @@ CG_DECL(20) CG_DECL(22) CG_DECL(24) CG_DECL(26) CG_DECL(28) CG_DECL(30) CG_DECL(
 
 bool gridding_supported(int d, int W) { return d >= 1 && d <= 3 && W >= 4 && W <= 32 && (W % 2) == 0; }
 
+// Constants of the fixed-point gridding.  vbits: a node's sum is at most 2^vbits times the
+// product of the largest tap sums S_t per dimension, which has to stay below 2^62, and each
+// sum before the last dimension below 2^58, where its high limb still has 31 bits.
+FixPar fix_params(const Geom& g) {
+  FixPar fp{};
+  double all = 0.0, last = 0.0;
+  for (int t = 0; t < g.d; ++t) {
+    const long double c = 1.0L / (logl(2.0L) * (long double)g.b[t]);
+    fp.c60[t] = (uint64_t)llrintl(ldexpl(c, 60));
+    fp.c57[t] = (int64_t)llrintl(ldexpl(c, kFixExpFrac));
+    fp.es_b2[t] = (double)((long double)g.es_beta[t] / logl(2.0L));
+    double most = 0.0;
+    for (int i = 0; i <= 16; ++i) {
+      double s = 0.0;
+      for (int l = 0; l < g.W; ++l) {
+        const double y = i / 16.0 + g.m - l, z = 1.0 - y * y * g.es_ia2;
+        s += g.window == kWinES ? (z > 0.0 ? exp(g.es_beta[t] * (sqrt(z) - 1.0)) : 0.0) : exp(-y * y / g.b[t]);
+      }
+      most = s > most ? s : most;
+    }
+    last = log2(1.02 * most);  // between the sampled fractions the sum hardly moves
+    all += last;
+  }
+  const int a = (int)floor(62.0 - all), b = (int)floor(58.0 - (all - last));
+  fp.vbits = a < b ? a : b;
+  if (fp.vbits > 55) fp.vbits = 55;
+  return fp;
+}
+
 // Larger of the interpolation and spreading kernels' shared-memory needs.
 size_t gridding_smem_bytes(const Plan& p) {
   const int d = p.geo.d, W = p.geo.W;
-  const size_t real = p.prec == kF64 ? 8 : 4;
+  if (p.prec == kF64) {
+    if (d == 3 && W > kFixWholeW) return 0;  // the planes go through in slabs
+    const size_t a = fix_smem_bytes(d, W, p.tl.E[0], false), b = fix_smem_bytes(d, W, p.tl.E[0], true);
+    return a > b ? a : b;
+  }
+  const size_t real = 4;
   const int nwarps = p.tl.threads / 32;
   const size_t a = grid_extra_smem(d, W, real, nwarps, p.tl.smem_tile, false);
   const size_t b = grid_extra_smem(d, W, real, nwarps, p.tl.smem_tile, true);

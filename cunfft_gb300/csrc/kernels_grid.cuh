@@ -1,4 +1,5 @@
-// kernels_grid.cuh -- tiled Gaussian gridding: interpolation (forward) and spreading (adjoint).
+// kernels_grid.cuh -- tiled Gaussian gridding: interpolation (forward) and spreading (adjoint)
+// of the FP32 form (the FP64 form's kernels are in kernels_fix.cuh).
 //
 // Method (the reference's, src/cunfft_kernel.cu:514-1149): node j touches the
 // (2m+2)^d grid points (u_t + l_t) mod n_t, l_t = 0..2m+1, with weight
@@ -95,23 +96,13 @@ __device__ __forceinline__ double2 cmul_add(double2 acc, double w, double2 v) {
   acc.y = fma(w, v.y, acc.y);
   return acc;
 }
-// A weight ready for the complex multiply-add: the (w, w) pair of a packed
-// f32x2 FMA in the FP32 form, the scalar in the FP64 form.
+// A weight ready for the complex multiply-add: the (w, w) pair of a packed f32x2 FMA.
 template <typename T> struct WPair;
 template <> struct WPair<float> {
   using t = float2;
   static __device__ __forceinline__ float2 make(float w) { return make_float2(w, w); }
 };
-template <> struct WPair<double> {
-  using t = double;
-  static __device__ __forceinline__ double make(double w) { return w; }
-};
 __device__ __forceinline__ float2 cmul_addp(float2 acc, float2 ww, float2 v) { return __ffma2_rn(ww, v, acc); }
-__device__ __forceinline__ double2 cmul_addp(double2 acc, double w, double2 v) {
-  acc.x = fma(w, v.x, acc.x);
-  acc.y = fma(w, v.y, acc.y);
-  return acc;
-}
 
 // Asynchronous global -> shared copy of one complex element (cp.async, 8 or 16 bytes).
 template <typename C>
@@ -574,6 +565,78 @@ __global__ void __launch_bounds__(512) k_spread(const typename Cx<T>::t* __restr
     }
     flush_tile<D, W, C>(tile, g + o.inst * geo.ntot, geo, tl, o);
     __syncthreads();
+  }
+}
+
+// One node through global memory: interpolation of the grid at the node (out[idx] written)
+// or its sample added to the grid with atomics.  off: the packed tile-local window start,
+// fr: the node's D fractions.
+template <int D, typename T, bool SPREAD>
+__device__ __forceinline__ void grid_node_global(const typename Cx<T>::t* __restrict__ in,
+                                                 typename Cx<T>::t* __restrict__ out, const Geom& geo,
+                                                 const TileOrigin& o, int idx, uint32_t off,
+                                                 const T* __restrict__ fr) {
+  using C = typename Cx<T>::t;
+  const int W = geo.W;
+  const T norm = (T)geo.norm;
+  int64_t s[kMaxDim];
+  T w[kMaxDim][kMaxTaps];
+  for (int t = 0; t < D; ++t) {
+    s[t] = o.a[t] + ((off >> (off_bits(D) * t)) & ((1u << off_bits(D)) - 1u));
+    WeightMath<T>::taps(fr[t], geo.m, geo, t, W, w[t]);
+  }
+  const int64_t inst_base = o.inst * geo.ntot;
+  if (!SPREAD) {
+    C acc;
+    acc.x = (T)0;
+    acc.y = (T)0;
+    for (int l0 = 0; l0 < W; ++l0) {
+      const int64_t i0 = wrap_up(s[0] + l0, geo.n[0]);
+      if (D == 1) {
+        acc = cmul_add(acc, w[0][l0], in[inst_base + i0]);
+        continue;
+      }
+      C a1;
+      a1.x = (T)0;
+      a1.y = (T)0;
+      for (int l1 = 0; l1 < W; ++l1) {
+        const int64_t i1 = wrap_up(s[1] + l1, geo.n[1]);
+        if (D == 2) {
+          a1 = cmul_add(a1, w[1][l1], in[inst_base + i0 * geo.n[1] + i1]);
+          continue;
+        }
+        C a2;
+        a2.x = (T)0;
+        a2.y = (T)0;
+        const int64_t rowb = inst_base + (i0 * geo.n[1] + i1) * geo.n[D - 1];
+        for (int l2 = 0; l2 < W; ++l2)
+          a2 = cmul_add(a2, w[D - 1][l2], in[rowb + wrap_up(s[D - 1] + l2, geo.n[D - 1])]);
+        a1 = cmul_add(a1, w[1][l1], a2);
+      }
+      acc = cmul_add(acc, w[0][l0], a1);
+    }
+    out[idx] = cscale(acc, norm);
+  } else {
+    const C v = cscale(in[idx], norm);
+    for (int l0 = 0; l0 < W; ++l0) {
+      const int64_t i0 = wrap_up(s[0] + l0, geo.n[0]);
+      const C v0 = cscale(v, w[0][l0]);
+      if (D == 1) {
+        global_add(&out[inst_base + i0], v0);
+        continue;
+      }
+      for (int l1 = 0; l1 < W; ++l1) {
+        const int64_t i1 = wrap_up(s[1] + l1, geo.n[1]);
+        const C v1 = cscale(v0, w[1][l1]);
+        if (D == 2) {
+          global_add(&out[inst_base + i0 * geo.n[1] + i1], v1);
+          continue;
+        }
+        const int64_t rowb = inst_base + (i0 * geo.n[1] + i1) * geo.n[D - 1];
+        for (int l2 = 0; l2 < W; ++l2)
+          global_add(&out[rowb + wrap_up(s[D - 1] + l2, geo.n[D - 1])], cscale(v1, w[D - 1][l2]));
+      }
+    }
   }
 }
 

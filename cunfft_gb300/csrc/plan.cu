@@ -105,7 +105,18 @@ static void default_tiles(const Plan* p, int* T) {
   const int d = p->geo.d, W = p->geo.W;
   // 2D FP32 with 2m+2 <= 16: 64 x 64 tiles, the largest the tensor-core spreading covers
   // (E0 = 63 + W rows of its 128-row MMA)
-  T[0] = d == 1 ? 2048 : (d == 2 ? (p->prec == kF32 && W <= 16 ? 64 : 32) : (p->prec == kF32 ? 8 : 4));
+  T[0] = d == 1 ? 2048 : (d == 2 ? (p->prec == kF32 && W <= 16 ? 64 : 32) : 8);
+  if (p->prec == kF64) {
+    if (d == 1) {
+      // small tiles: clearing and adding out a tile costs little beside its nodes; larger
+      // ones where there would be very many
+      T[0] = 256;
+      while (T[0] < 1024 && p->geo.n[0] / T[0] * p->geo.batch > 16384) T[0] *= 2;
+    }
+    if (d >= 2) T[d - 1] = fix_t_last(d);
+    if (d == 3) T[1] = fix_t_mid(d);
+    return;
+  }
   if (d == 2) T[1] = fixed_t_last(2, W);
   if (d == 3) {
     T[1] = fixed_t_mid(3, W);
@@ -123,8 +134,10 @@ static Tiling make_tiling(const Plan* p, const int* T, int chunk) {
   }
   // inner strides are the kernels' compile-time values (inner tiles may be
   // smaller than the fixed extents when the grid is small)
-  int64_t elems;
-  if (d == 1) {
+  int64_t elems = 0;
+  if (p->prec == kF64) {
+    // kernels_fix.cuh has its own strides and sizes its shared memory itself
+  } else if (d == 1) {
     tl.S = tl.E[0];
     tl.R1 = 1;
     elems = tl.S;
@@ -148,7 +161,8 @@ static Tiling make_tiling(const Plan* p, const int* T, int chunk) {
   // CTAs better.  On the batched 2D workload 512 and 256 spread equally fast, 256 at 0.64
   // times the error against the FP64 form.
   const bool t2 = d == 2 && p->prec == kF32 && W <= 16;
-  tl.chunk = chunk > 0 ? chunk : (d == 3 ? 1024 : (t2 ? 256 : 2048));
+  // FP64 (fixed point): 512 nodes leave a cell's sum 53 bits below the largest sample
+  tl.chunk = chunk > 0 ? chunk : (p->prec == kF64 ? 512 : (d == 3 ? 1024 : (t2 ? 256 : 2048)));
   tl.use_global = 0;
   tl.ns = 1;  // no sub-bins unless the plan asks for them (plan_choose_tiling)
   return tl;
@@ -387,6 +401,7 @@ int geom_init(Plan* p, int d, const int64_t* N, const int64_t* n, int m, int pre
   }
   if (g.ntot * batch >= ((int64_t)1 << 40)) return set_status(p, CUNFFT_X_INVALID_ARGUMENT, "grid too large");
   window_constants(g, kWinGauss);
+  p->fix = fix_params(g);
   p->prec = prec;
   CG_TRY(check_cuda(p, cudaGetDevice(&p->device), "cudaGetDevice"));
   CG_TRY(check_cuda(p, cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device),
@@ -404,6 +419,7 @@ int plan_set_window(Plan* p, int window) {
   if (window != p->geo.window) {
     CG_TRY(check_cuda(p, cudaStreamSynchronize(p->stream), "cudaStreamSynchronize"));  // the old table may be in use
     window_constants(p->geo, window);
+    p->fix = fix_params(p->geo);
     const std::vector<double> tab = roc_factors(p->geo);
     CG_TRY(check_cuda(p, cudaMemcpy(p->roc_tab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice),
                       "upload roll-off table"));

@@ -36,6 +36,7 @@ struct Plan {
   bool own_g = false;
   double* roc_tab = nullptr;   // per-dim roll-off factors 1 / phi_hat_t(k_t / n_t), sum_t N_t doubles
   Tiling tl{};
+  FixPar fix{};                // FP64 form: constants of the fixed-point gridding (fix_params)
   Bins bins{};
   int64_t bins_capacity_M = -1;
   int64_t bins_capacity_tiles = -1;
@@ -165,6 +166,7 @@ cudaError_t launch_ndft_forward(const Plan& p, const double* x, const void* fhat
 cudaError_t launch_ndft_adjoint(const Plan& p, const double* x, const void* f, void* fhat, cudaStream_t st,
                                 const int64_t* kidx = nullptr, int64_t nsel = 0);
 size_t gridding_smem_bytes(const Plan& p);
+FixPar fix_params(const Geom& g);
 int gridding_max_smem(const Plan& p);
 bool gridding_supported(int d, int W);
 
