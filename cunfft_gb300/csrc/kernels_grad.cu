@@ -8,9 +8,12 @@
 // FFT'd grid g as the forward transform and contracts them with the incoming
 // gradient: grad_x[j, t] = Re(conj(grad_f_j) * d f_j / d x_{j,t}).
 // No reference counterpart (the reference has no differentiable transform).
-// One thread per node, FP64 node reduction and weights, grid read through L1/L2;
-// accumulation in the plan's real type.
-#include "runtime.h"
+// FP64 node reduction and weights; accumulation in the plan's real type.  The FP32 form runs
+// on staged tiles (kernels_grad_tile.cuh); the kernel here, one thread per node with the
+// grid read through L1/L2, takes the FP64 form and tiles that do not fit in shared memory.
+#include <math.h>
+
+#include "kernels_grad_tile.cuh"
 
 namespace cg {
 
@@ -98,8 +101,35 @@ __global__ void __launch_bounds__(128) k_interp_grad(const double* __restrict__ 
   }
 }
 
+#define CG_DECL(W) \
+  cudaError_t grid_grad_w##W(const Plan&, const GradPar&, const void*, const void*, double*, cudaStream_t);
+CG_DECL(4) CG_DECL(6) CG_DECL(8) CG_DECL(10) CG_DECL(12) CG_DECL(14) CG_DECL(16) CG_DECL(18)
+CG_DECL(20) CG_DECL(22) CG_DECL(24) CG_DECL(26) CG_DECL(28) CG_DECL(30) CG_DECL(32)
+#undef CG_DECL
+
+static cudaError_t launch_grad_tile(const Plan& p, const void* g, const void* grad_f, double* grad_x, cudaStream_t st) {
+  GradPar gp{};
+  for (int t = 0; t < p.geo.d; ++t) {
+    int e;
+    const double f = frexp(2.0 / p.geo.b[t] * (double)p.geo.n[t], &e);  // f in [1/2, 1)
+    gp.mant[t] = (uint64_t)ldexp(f, 63);
+    gp.scale[t] = -(float)ldexp(1.0, e - 60);  // the kernel's product: w |y| 2^61 f 2^63 / 2^64
+  }
+  const cudaError_t e = cudaMemsetAsync(p.bins.work, 0, sizeof(int32_t), st);
+  if (e != cudaSuccess) return e;
+  switch (p.geo.W) {
+#define CG_CASE(W) case W: return grid_grad_w##W(p, gp, g, grad_f, grad_x, st);
+    CG_CASE(4) CG_CASE(6) CG_CASE(8) CG_CASE(10) CG_CASE(12) CG_CASE(14) CG_CASE(16) CG_CASE(18)
+    CG_CASE(20) CG_CASE(22) CG_CASE(24) CG_CASE(26) CG_CASE(28) CG_CASE(30) CG_CASE(32)
+#undef CG_CASE
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 cudaError_t launch_interp_grad(const Plan& p, const void* g, const void* grad_f, double* grad_x, cudaStream_t st) {
   if (p.M == 0) return cudaSuccess;
+  // the shared-tile kernels' shared memory covers the tile and more than the exponential's table
+  if (p.prec == kF32 && !p.tl.use_global) return launch_grad_tile(p, g, grad_f, grad_x, st);
   int64_t b = (p.M + 127) / 128;
   if (b > (int64_t)p.num_sms * 16) b = (int64_t)p.num_sms * 16;
   if (p.prec == kF64)

@@ -753,6 +753,7 @@ int plan_ndft_adjoint(Plan* p, const void* f, void* fhat, const int64_t* kidx, i
 
 int plan_node_gradient(Plan* p, const void* fhat, const void* grad_f, double* grad_x) {
   if (!p->nodes_set) return set_status(p, CUNFFT_X_NODES_NOT_SET, "gradient: nodes not set");
+  if (!p->bins.valid) CG_TRY(rebin(p));
   CG_TRY(check_cuda(p, launch_roc_forward(*p, fhat, p->g, p->stream), "roll-off kernel"));
   CG_TRY(check_cufft(p, exec_fft(p, p->fft, p->g, CUFFT_FORWARD), "forward FFT"));
   CG_TRY(check_cuda(p, launch_interp_grad(*p, p->g, grad_f, grad_x, p->stream), "gradient kernel"));
