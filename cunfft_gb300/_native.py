@@ -87,7 +87,7 @@ X_SYMBOLS = [
     "cunfft_x_spread_noalloc", "cunfft_x_set_spread_kernel", "cunfft_x_get_spread_kernel",
     "cunfft_x_set_window", "cunfft_x_get_window",
     "cunfft_x_set_interp_kernel", "cunfft_x_get_interp_kernel", "cunfft_x_forward_host", "cunfft_x_adjoint_host",
-    "cunfft_x_check_wait_timeout",
+    "cunfft_x_check_wait_timeout", "cunfft_x_cg",
 ]
 UTIL_SYMBOLS = [
     "showTimes", "getGPUMemProps_ToStdout", "showCPUMemUse", "showCoeff_double", "showCoeff_cuComplex",
@@ -125,6 +125,8 @@ def lib():
         "cunfft_x_ndft_adjoint": (ctypes.c_int, [vp, vp, vp]),
         "cunfft_x_ndft_adjoint_at": (ctypes.c_int, [vp, vp, vp, ctypes.c_int64, vp]),
         "cunfft_x_node_gradient": (ctypes.c_int, [vp, vp, vp, vp]),
+        "cunfft_x_cg": (ctypes.c_int, [vp, ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_double, ctypes.c_double,
+                                       vp, vp, vp, vp, vp, vp, vp]),
         "cunfft_x_interp": (ctypes.c_int, [vp, vp, vp]),
         "cunfft_x_spread": (ctypes.c_int, [vp, vp, vp]),
         "cunfft_x_set_stream": (ctypes.c_int, [vp, vp]),

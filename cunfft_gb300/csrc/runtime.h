@@ -165,6 +165,8 @@ cudaError_t launch_interp_grad(const Plan& p, const void* g, const void* grad_f,
 cudaError_t launch_ndft_forward(const Plan& p, const double* x, const void* fhat, void* f, cudaStream_t st);
 cudaError_t launch_ndft_adjoint(const Plan& p, const double* x, const void* f, void* fhat, cudaStream_t st,
                                 const int64_t* kidx = nullptr, int64_t nsel = 0);
+cudaError_t launch_cg(const Plan& p, int stage, int64_t it, int64_t iters, double lam, double tol, const void* b, void* x,
+                      void* r, void* pv, void* ap, double* scal, int32_t* stop, cudaStream_t st);
 size_t gridding_smem_bytes(const Plan& p);
 FixPar fix_params(const Geom& g);
 int gridding_max_smem(const Plan& p);

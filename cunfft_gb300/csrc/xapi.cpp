@@ -79,6 +79,16 @@ int cunfft_x_node_gradient(cunfft_x_plan* h, const void* fhat, const void* grad_
   return cg::plan_node_gradient(&h->p, fhat, grad_f, grad_x);
 }
 
+int cunfft_x_cg(cunfft_x_plan* h, int stage, int64_t it, int64_t iters, double lam, double tol, const void* b, void* x,
+                void* r, void* p, void* ap, double* scal, int32_t* stop) {
+  if (!h || stage < CUNFFT_X_CG_BEGIN || stage > CUNFFT_X_CG_TURN || iters < 1 || it < 0 || it >= iters || !b || !x || !r ||
+      !p || !ap || !scal || !stop)
+    return CUNFFT_X_INVALID_ARGUMENT;
+  const int s = cg::check_cuda(&h->p, cg::launch_cg(h->p, stage, it, iters, lam, tol, b, x, r, p, ap, scal, stop, h->p.stream),
+                               "conjugate gradient kernel");
+  return s != CUNFFT_X_SUCCESS ? s : cg::set_status(&h->p, CUNFFT_X_SUCCESS, nullptr);
+}
+
 int cunfft_x_interp(cunfft_x_plan* h, const void* g, void* f) {
   if (!h) return CUNFFT_X_INVALID_ARGUMENT;
   return cg::plan_interp_only(&h->p, g, f);

@@ -10,9 +10,13 @@ of the first kind,
 
 with optional sample weights W (e.g. density compensation) and Tikhonov term
 lam.  Every iteration costs one forward and one adjoint NFFT on the plan's
-nodes; the vector algebra runs as torch operations on the same stream.
+nodes; the vector algebra is three kernels on the same stream with their scalars on the
+device, so the host waits once at the end (every iteration with a callback or a tolerance).
 """
 import torch
+
+from . import _native as nat
+from .nfft import _ptr
 
 
 def cgne(plan, f, iters=20, weights=None, lam=0.0, fhat0=None, tol=0.0, callback=None):
@@ -27,35 +31,48 @@ def cgne(plan, f, iters=20, weights=None, lam=0.0, fhat0=None, tol=0.0, callback
     f = f.to(cd)
     w = None if weights is None else weights.to(f.real.dtype)
     shape = plan._coef_shape()
+    iters = int(iters)
 
-    def normal_op(v):
-        av = plan.forward(v)
-        if w is not None:
-            av = av * w
-        out = plan.adjoint(av)
-        if lam:
-            out = out + lam * v
-        return out
+    def normal_op(v, out=None, samples=None):
+        av = plan.forward(v, out=samples)
+        return plan.adjoint(av * w if w is not None else av, out=out)
 
     b = plan.adjoint(f * w if w is not None else f)
-    x = torch.zeros(shape, dtype=cd, device=f.device) if fhat0 is None else fhat0.to(cd).clone()
-    r = b - normal_op(x) if fhat0 is not None else b.clone()
-    p = r.clone()
-    rr = torch.vdot(r.reshape(-1), r.reshape(-1)).real
-    bnorm = torch.linalg.norm(b.reshape(-1))
+    x = torch.zeros(shape, dtype=cd, device=f.device) if fhat0 is None else fhat0.to(cd).clone().contiguous()
+    r = b.clone()
+    if fhat0 is not None:
+        r -= normal_op(x)
+        if lam:
+            r -= lam * x
+    if iters < 1:
+        return x, []
+    p, ap = r.clone(), torch.empty_like(r)
+    samples = torch.empty_like(f)
+    # every scalar stays on the device: <b, b>, <r, r> and <p, ap> per iteration, the history
+    scal = torch.zeros(2 + 3 * iters, dtype=torch.float64, device=f.device)
+    stop = torch.zeros(iters + 1, dtype=torch.int32, device=f.device)
+    args = [_ptr(t) for t in (b, x, r, p, ap, scal, stop)]
+
+    def stage(kind, it):
+        nat.check(plan._lib.cunfft_x_cg(plan._h, kind, it, iters, float(lam), float(tol), *args), plan._h)
+
+    stage(0, 0)
+    wait = callback is not None or tol > 0.0
     hist = []
-    for _ in range(int(iters)):
-        ap = normal_op(p)
-        alpha = rr / torch.vdot(p.reshape(-1), ap.reshape(-1)).real
-        x = x + alpha * p
-        r = r - alpha * ap
-        rr_new = torch.vdot(r.reshape(-1), r.reshape(-1)).real
-        rel = (torch.sqrt(rr_new) / bnorm).item()
-        hist.append(rel)
-        if callback is not None:
-            callback(x, rel)
-        if rel <= tol:
-            break
-        p = r + (rr_new / rr) * p
-        rr = rr_new
+    for it in range(iters):
+        normal_op(p, out=ap, samples=samples)
+        stage(1, it)
+        stage(2, it)
+        stage(3, it)
+        if wait:
+            rel = scal[2 + 2 * iters + it].item()
+            hist.append(rel)
+            if callback is not None:
+                callback(x.clone(), rel)
+            if rel <= tol:
+                break
+    if not wait:
+        hist = scal[2 + 2 * iters:].tolist()
+        if 0.0 in hist:  # solved exactly: the iterations after it changed nothing
+            del hist[hist.index(0.0) + 1:]
     return x, hist

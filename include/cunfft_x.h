@@ -122,6 +122,24 @@ int cunfft_x_ndft_adjoint_at(cunfft_x_plan *plan, const void *f, const int64_t *
  *  forward transform.  grad_x is a device array of sum_i M_i * d doubles. */
 int cunfft_x_node_gradient(cunfft_x_plan *plan, const void *f_hat, const void *grad_f, double *grad_x);
 
+/* Vector algebra of conjugate gradients on (A^H W A + lam I) x = b, one launch per call on
+ * the plan's stream, vectors of batch N_total coefficients in the plan's precision, all
+ * scalars in device memory: scal holds 2 + 3 iters doubles (<b, b>; <r, r> of iterations
+ * 0 .. iters; Re <p, ap> and the relative residual of iterations 0 .. iters - 1) and stop
+ * iters + 1 flags, both zeroed by the caller before
+ *   CUNFFT_X_CG_BEGIN  <b, b> and <r, r>;
+ * and then, per iteration `it`, with ap = A^H W A p formed by the caller,
+ *   CUNFFT_X_CG_DOT    ap += lam p and Re <p, ap>,
+ *   CUNFFT_X_CG_STEP   x += alpha p, r -= alpha ap and <r, r>,
+ *   CUNFFT_X_CG_TURN   p = r + beta p, the relative residual sqrt(<r, r> / <b, b>) and
+ *                      stop[it + 1] when it is at most tol: later iterations change nothing. */
+#define CUNFFT_X_CG_BEGIN 0
+#define CUNFFT_X_CG_DOT 1
+#define CUNFFT_X_CG_STEP 2
+#define CUNFFT_X_CG_TURN 3
+int cunfft_x_cg(cunfft_x_plan* plan, int stage, int64_t it, int64_t iters, double lam, double tol, const void* b, void* x,
+                void* r, void* p, void* ap, double* scal, int32_t* stop);
+
 /** Gridding stages alone, on a caller-provided oversampled grid g
  *  (batch*n_total complex, plan precision): interpolation g -> f and
  *  spreading f -> g (spreading accumulates into g; clear it first).  g needs only
