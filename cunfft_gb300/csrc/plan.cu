@@ -476,6 +476,7 @@ int plan_init(Plan* p, int d, const int64_t* N, const int64_t* n, int m, int pre
     }
     p->fft = h;
     p->own_fft = true;
+    fft_fix_prepare(*p);
   }
   // per-instance node offsets, status flag, work counters
   CG_TRY(check_cuda(p, plan_malloc(&p->bins.inst_off, sizeof(int32_t) * (batch + 1)), "cudaMalloc"));
@@ -517,6 +518,7 @@ void plan_release(Plan* p) {
   p->g = nullptr;
   cudaFree(p->roc_tab);
   p->roc_tab = nullptr;
+  fft_fix_release(*p);
   if (p->own_fft && p->fft) cufftDestroy(p->fft);
   p->fft = 0;
   for (int i = 0; i < 8; ++i)
@@ -633,6 +635,19 @@ static cufftResult exec_fft(const Plan* p, cufftHandle h, void* data, int dir) {
   return cufftExecC2C(h, (cufftComplex*)data, (cufftComplex*)data, dir);
 }
 
+// Roll-off, zero padding and forward FFT of the coefficients into the grid.  The FP64 form's
+// FFT does all three; its time counts as the FFT's.
+static void rec(Plan* p, int i);
+static int forward_grid(Plan* p, const void* fhat, cufftHandle h) {
+  if (p->fx_on) {
+    rec(p, 1);
+    return check_cuda(p, launch_fft_fix(*p, fhat, p->g, false, p->stream), "forward FFT");
+  }
+  CG_TRY(check_cuda(p, launch_roc_forward(*p, fhat, p->g, p->stream), "roll-off kernel"));
+  rec(p, 1);
+  return check_cufft(p, exec_fft(p, h, p->g, CUFFT_FORWARD), "forward FFT");
+}
+
 static void rec(Plan* p, int i) {
   if (p->timing) cudaEventRecord(p->ev[i], p->stream);
 }
@@ -659,9 +674,7 @@ int plan_forward(Plan* p, const void* fhat, void* f) {
   CG_TRY(prepare_interp(p));
   if (p->timing) p->last_dir = 0;
   rec(p, 0);
-  CG_TRY(check_cuda(p, launch_roc_forward(*p, fhat, p->g, p->stream), "roll-off kernel"));
-  rec(p, 1);
-  CG_TRY(check_cufft(p, exec_fft(p, p->fft_fwd_ext ? p->fft_fwd_ext : p->fft, p->g, CUFFT_FORWARD), "forward FFT"));
+  CG_TRY(forward_grid(p, fhat, p->fft_fwd_ext ? p->fft_fwd_ext : p->fft));
   rec(p, 2);
   CG_TRY(check_cuda(p, launch_interp(*p, p->g, f, p->stream), "interpolation kernel"));
   rec(p, 3);
@@ -677,7 +690,10 @@ int plan_adjoint(Plan* p, const void* f, void* fhat) {
                     "clear grid"));
   CG_TRY(check_cuda(p, launch_spread(*p, f, p->g, p->stream), "spreading kernel"));
   rec(p, 1);
-  CG_TRY(check_cufft(p, exec_fft(p, p->fft_bwd_ext ? p->fft_bwd_ext : p->fft, p->g, CUFFT_INVERSE), "adjoint FFT"));
+  if (p->fx_on)
+    CG_TRY(check_cuda(p, launch_fft_fix(*p, nullptr, p->g, true, p->stream), "adjoint FFT"));
+  else
+    CG_TRY(check_cufft(p, exec_fft(p, p->fft_bwd_ext ? p->fft_bwd_ext : p->fft, p->g, CUFFT_INVERSE), "adjoint FFT"));
   rec(p, 2);
   CG_TRY(check_cuda(p, launch_roc_adjoint(*p, p->g, fhat, p->stream), "roll-off kernel"));
   rec(p, 3);
@@ -754,8 +770,13 @@ int plan_ndft_adjoint(Plan* p, const void* f, void* fhat, const int64_t* kidx, i
 int plan_node_gradient(Plan* p, const void* fhat, const void* grad_f, double* grad_x) {
   if (!p->nodes_set) return set_status(p, CUNFFT_X_NODES_NOT_SET, "gradient: nodes not set");
   if (!p->bins.valid) CG_TRY(rebin(p));
-  CG_TRY(check_cuda(p, launch_roc_forward(*p, fhat, p->g, p->stream), "roll-off kernel"));
-  CG_TRY(check_cufft(p, exec_fft(p, p->fft, p->g, CUFFT_FORWARD), "forward FFT"));
+  {
+    const bool timing = p->timing;  // the stage times stay those of the last transform
+    p->timing = false;
+    const int s = forward_grid(p, fhat, p->fft);
+    p->timing = timing;
+    if (s != CUNFFT_X_SUCCESS) return s;
+  }
   CG_TRY(check_cuda(p, launch_interp_grad(*p, p->g, grad_f, grad_x, p->stream), "gradient kernel"));
   return set_status(p, CUNFFT_X_SUCCESS, nullptr);
 }

@@ -30,6 +30,12 @@ struct Plan {
   bool own_stream = false;
   cufftHandle fft = 0;         // batched plan used for both directions
   bool own_fft = false;
+  // FP64 form: twiddle tables and 1D scratch of the fixed-point FFT (kernels_fft.cu); off:
+  // the library's FFT
+  int4* fx_tab = nullptr;
+  void* fx_tmp = nullptr;
+  int64_t fx_off[4] = {0, 0, 0, 0};
+  bool fx_on = false;
   cufftHandle fft_fwd_ext = 0; // handles lent by the drop-in ABI (0: use fft)
   cufftHandle fft_bwd_ext = 0;
   void* g = nullptr;           // batch * ntot complex
@@ -158,6 +164,9 @@ void interp_tc_release(Plan& p);
 // launchers (kernel .cu files); all asynchronous on st
 cudaError_t launch_binning(const Plan& p, const double* x, cudaStream_t st);
 cudaError_t launch_roc_forward(const Plan& p, const void* fhat, void* g, cudaStream_t st);
+cudaError_t launch_fft_fix(const Plan& p, const void* fhat, void* g, bool inv, cudaStream_t st);
+void fft_fix_prepare(Plan& p);
+void fft_fix_release(Plan& p);
 cudaError_t launch_roc_adjoint(const Plan& p, const void* g, void* fhat, cudaStream_t st);
 cudaError_t launch_interp(const Plan& p, const void* g, void* f, cudaStream_t st);
 cudaError_t launch_spread(const Plan& p, const void* f, void* g, cudaStream_t st);
