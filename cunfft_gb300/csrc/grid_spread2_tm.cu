@@ -2,6 +2,7 @@
 // (kernels_spread2_tm.cuh).
 #include <algorithm>
 
+#include "kernels_spread2_sub.cuh"
 #include "kernels_spread2_tm.cuh"
 
 namespace cg {
@@ -15,9 +16,31 @@ bool spread2_tm_supported(const Plan& p) {
 // never waits.
 static constexpr size_t kT2SmemFloor = 228u * 1024u / 2u + 1u;
 
+// The sub-tile kernel, where the binning makes its items.  Its items cost about as much with
+// few nodes as with many, so a grid of many sub-tiles with only a few nodes each goes to the
+// whole-tile kernel.  Measured (m = 6; us, sub-tile / whole-tile): n = 1024^2 (4096 sub-tiles)
+// M = 1000 13 / 19, 10^4 28 / 22, 5 10^4 30 / 33, 2 10^5 37 / 83; n = 256^2 M = 1000 11 / 19,
+// 2 10^5 28 / 76.
+static bool use_sub(const Plan& p) {
+  if (!p.tl.sub_on || !p.tl.sub_items) return false;
+  const int64_t keys = p.tl.tiles_total * p.tl.ns;
+  return p.bins.M >= 8 * keys || std::min(p.bins.M, keys) <= (int64_t)2 * p.num_sms * kS2PerSm;
+}
+
+template <int W>
+static cudaError_t launch_sub(const Plan& p, const void* in, void* out, cudaStream_t st) {
+  auto kern = p.geo.window == kWinES ? k_spread2_sub<W, kWinES> : k_spread2_sub<W, kWinGauss>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kS2Smem);
+  if (e != cudaSuccess) return e;
+  // (the occupancy call counts one CTA per SM for a kernel that allocates tensor memory)
+  kern<<<p.num_sms * kS2PerSm, kS2Threads, kS2Smem, st>>>((const float2*)in, (float2*)out, p.geo, p.tl, p.bins);
+  return cudaGetLastError();
+}
+
 template <int W>
 static cudaError_t launch_t2(const Plan& p, const void* in, void* out, cudaStream_t st) {
   if (!spread2_tm_supported(p)) return cudaErrorInvalidConfiguration;
+  if (use_sub(p)) return launch_sub<W>(p, in, out, st);
   const size_t smem = std::max<size_t>(t2_layout().total, kT2SmemFloor);
   auto kern = p.geo.window == kWinES ? k_spread2_tm<W, kWinES> : k_spread2_tm<W, kWinGauss>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
