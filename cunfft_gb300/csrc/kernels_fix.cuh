@@ -44,6 +44,12 @@ __host__ __device__ constexpr int fix_interp_warps(int d) { return d == 3 ? 16 :
 __host__ __device__ constexpr int fix_nodes_per_warp(int d) { return d == 1 ? 32 : (d == 3 ? 2 : 8); }
 __host__ __device__ constexpr int fix_spread_warps(int d) { return d == 3 ? 16 : (d == 2 ? 8 : 4); }
 __host__ __device__ constexpr int fix_batch(int d) { return d == 3 ? 20 : 64; }
+// CTAs per SM the registers are limited for: in 1D and 2D an item is a few short phases
+// between barriers, which other CTAs fill (2D, m = 6, M = 2^18: spreading 252 -> 223 us,
+// interpolation 149 -> 140 us)
+__host__ __device__ constexpr int fix_ctas(int d, int W, bool spread) {
+  return d == 3 || W > 16 ? 1 : (spread && d == 2 ? 3 : 4);
+}
 // 1D spreading: node groups per warp (two windows of W <= 16 taps side by side)
 __host__ __device__ constexpr int fix_spread_groups(int W) { return W <= 16 ? 2 : 1; }
 // d = 3: up to this many taps the whole padded tile of 8 window starts fits in shared
@@ -179,7 +185,7 @@ struct BoolC {
 };
 
 template <int D, int W, bool SLAB>
-__global__ void __launch_bounds__(fix_interp_warps(D) * 32, 1)
+__global__ void __launch_bounds__(fix_interp_warps(D) * 32, fix_ctas(D, W, false))
     k_interp_fix(const double2* __restrict__ g, double2* __restrict__ f, Geom geo, Tiling tl, Bins bins, FixPar fp) {
   constexpr int R = kWarp / W, NIT = (W + R - 1) / R;
   constexpr bool FULL = R * NIT == W;
@@ -461,7 +467,7 @@ __device__ __forceinline__ void fix_cells_add(longlong2* cells, int stride, cons
 }
 
 template <int D, int W, bool SLAB>
-__global__ void __launch_bounds__(fix_spread_warps(D) * 32, 1)
+__global__ void __launch_bounds__(fix_spread_warps(D) * 32, fix_ctas(D, W, true))
     k_spread_fix(const double2* __restrict__ f, double2* __restrict__ g, Geom geo, Tiling tl, Bins bins, FixPar fp) {
   constexpr int R = kWarp / W;
   constexpr int NBC = fix_batch(D), NW = fix_spread_warps(D);
