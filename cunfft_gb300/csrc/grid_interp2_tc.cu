@@ -39,8 +39,8 @@ bool interp2_tc_supported(const Plan& p) {
 }
 
 // Split rows half [batch][4][P0][P2s], row scales float [batch][P0], and the 5-D map over
-// the rows (dims P2s, P0, 1, component, instance; box 32 halves x (16 + W - 1) rows,
-// 64-byte swizzle, zero fill outside).  Box rows are 64 bytes (32 halves); rows of the
+// the rows (dims P2s, P0, 1, component, instance; box 32 halves x 32 rows x 4
+// components, 64-byte swizzle, zero fill outside).  Box rows are 64 bytes (32 halves); rows of the
 // arrays are multiples of 16 bytes (P2s % 8 == 0).
 cudaError_t interp2_tc_prepare(Plan& p, PFN_cuTensorMapEncodeTiled_v12000 enc) {
   if (p.it_ready) return cudaSuccess;
@@ -56,11 +56,10 @@ cudaError_t interp2_tc_prepare(Plan& p, PFN_cuTensorMapEncodeTiled_v12000 enc) {
       return e;
     }
   }
-  const int E0S = kI2Sub + p.geo.W - 1;  // rows of a 16-row sub-tile's windows (the kernel's B rows)
   const cuuint64_t dims[5] = {(cuuint64_t)sd.P2s, (cuuint64_t)sd.P0, 1u, 4u, (cuuint64_t)p.geo.batch};
   const cuuint64_t strides[4] = {(cuuint64_t)(sd.P2s * 2), (cuuint64_t)(comp * 2), (cuuint64_t)(comp * 2),
                                  (cuuint64_t)(4 * comp * 2)};
-  const cuuint32_t box[5] = {(cuuint32_t)kI2K, (cuuint32_t)E0S, 1u, 1u, 1u};
+  const cuuint32_t box[5] = {(cuuint32_t)kI2K, (cuuint32_t)kI2Rows, 1u, 4u, 1u};
   const cuuint32_t estr[5] = {1u, 1u, 1u, 1u, 1u};
   const CUresult r = enc(&p.it_tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, p.it_split, dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
