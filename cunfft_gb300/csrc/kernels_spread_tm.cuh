@@ -96,14 +96,32 @@ __host__ __device__ inline TmLayout tm_layout(int W, int E0) {
   return L;
 }
 
-// TcCursor step over batches of kTmK nodes
+// The item this CTA takes after item `it`: each round of G items goes to the G CTAs, five
+// places further on every time.  Taking items c, c + G, ... instead gives a CTA the same tile
+// columns over and over when G and the tiles of a row share a factor; 16 tiles of a row and
+// 152 CTAs then leave one CTA in eight with half of its tiles at the row's wrap (two bulk
+// reductions for each row), and those CTAs finished at 1.84 M cycles, the others at 1.55 M.
+__device__ __forceinline__ int tm_next_item(int it) {
+  const int G = (int)gridDim.x, k = it / G;
+  return (k + 1) * G + (it - k * G + 5) % G;
+}
+__device__ __forceinline__ int4 tm_item(const Bins& bins, int it, int num_items) {
+  return it < num_items ? bins.items[it] : make_int4(0, 0, 0, 0);
+}
+
+// TcCursor over batches of kTmK nodes of this CTA's items
+__device__ __forceinline__ void tm_cursor_init(TcCursor& c, const Bins& bins, int num_items) {
+  c.it = (int)blockIdx.x;
+  c.b = 0;
+  c.item = tm_item(bins, c.it, num_items);
+  c.next = tm_item(bins, tm_next_item(c.it), num_items);
+}
 __device__ __forceinline__ void tm_cursor_step(TcCursor& c, const Bins& bins, int num_items) {
-  const int G = (int)gridDim.x;
   if (c.item.y + (++c.b) * kTmK < c.item.z) return;
-  c.it += G;
+  c.it = tm_next_item(c.it);
   c.b = 0;
   c.item = c.next;
-  c.next = c.it + G < num_items ? bins.items[c.it + G] : make_int4(0, 0, 0, 0);
+  c.next = tm_item(bins, tm_next_item(c.it), num_items);
 }
 
 template <int W, int WIN>
@@ -127,7 +145,6 @@ __global__ void __launch_bounds__(kTmThreads, 1) k_spread_tm(const float2* __res
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.bar_off + 132);  // a wait gave up
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int num_items = *bins.num_items;
-  const int G = (int)gridDim.x;
 
   if (tid == 0) {
     for (int i = 0; i < 4; ++i) {
@@ -149,7 +166,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) k_spread_tm(const float2* __res
   const uint32_t tmem = *tmem_slot;
   bool healthy = true;
 
-  // Every role walks items c, c + G, ... (CTA c); batch gb (counted across the CTA's
+  // Every role walks the same items (tm_next_item); batch gb (counted across the CTA's
   // items) uses stage gb % 4 in its cycle gb / 4 and record / table buffers gb & 1.
   // A role whose bounded wait gives up raises abort_flag and leaves its loop; the
   // builders leave together after their barrier, the others at their next wait, so a
@@ -185,7 +202,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) k_spread_tm(const float2* __res
       }
     };
     TcCursor cc, lc;  // the batch being built and the batch being loaded
-    tc_cursor_init(cc, bins, num_items);
+    tm_cursor_init(cc, bins, num_items);
     lc = cc;
 #pragma unroll
     for (int d = 0; d < kTmRing - 1; ++d) {
@@ -204,11 +221,6 @@ __global__ void __launch_bounds__(kTmThreads, 1) k_spread_tm(const float2* __res
         tm_cursor_step(lc, bins, num_items);
       }
       cp_async_commit();
-      // stage st (its B buffer and its A columns) is free once the MMAs of batch gb - 4
-      // are complete: one thread waits, the barrier after phase (1) publishes it
-      bool fail = false;
-      if (cyc > 0 && tid == kBuildThreads - 32) fail = !tc::mbar_wait_bounded(&empty[st], (cyc - 1u) & 1u, kTcPolls);
-      healthy &= !fail;
       const unsigned char* sl = smem + L.rec_off + (gb % kTmRing) * kTmSlotBytes;
       const uint32_t* roff = reinterpret_cast<const uint32_t*>(sl + kTmSlotOff);
       const float* frac = reinterpret_cast<const float*>(sl + kTmSlotFrac);
@@ -253,6 +265,12 @@ __global__ void __launch_bounds__(kTmThreads, 1) k_spread_tm(const float2* __res
           }
         }
       }
+      // stage st (its B buffer and its A columns) is free once the MMAs of batch gb - 2
+      // are complete: one thread waits, after its tables, which do not need the stage; the
+      // barrier after phase (1) publishes it
+      bool fail = false;
+      if (cyc > 0 && tid == kBuildThreads - 32) fail = !tc::mbar_wait_bounded(&empty[st], (cyc - 1u) & 1u, kTcPolls);
+      healthy &= !fail;
       cp_async_wait_group<kTmRing - 2>();  // this thread's loads of batch gb + 1 have landed
       // (1) done; stage st free, tables and next records visible; the builders leave
       // together when any of them saw a wait give up or the abort flag raised
@@ -341,10 +359,10 @@ __global__ void __launch_bounds__(kTmThreads, 1) k_spread_tm(const float2* __res
       const uint64_t d_stage = (uint64_t)(kTmBStage >> 4);  // stage s = stage 0 + s d_stage
       const uint32_t idesc = tc::idesc_f16(128, kTcN);
       uint32_t gb = 0, st = 0, cyc = 0, k = 0;
-      int4 nxt = (int)blockIdx.x < num_items ? bins.items[blockIdx.x] : make_int4(0, 0, 0, 0);
-      for (int it = blockIdx.x; it < num_items; it += G, ++k) {
+      int4 nxt = tm_item(bins, blockIdx.x, num_items);
+      for (int it = blockIdx.x; it < num_items; it = tm_next_item(it), ++k) {
         const int4 item = nxt;
-        if (it + G < num_items) nxt = bins.items[it + G];  // one item ahead
+        nxt = tm_item(bins, tm_next_item(it), num_items);  // one item ahead
         const int nbatch = (item.z - item.y + kTmK - 1) / kTmK;
         for (int b = 0; b < nbatch && healthy; ++b, ++gb) {
           const int halves = item.z - (item.y + b * kTmK) > 16 ? 2 : 1;  // k-steps built (as the builders)
@@ -409,10 +427,10 @@ __global__ void __launch_bounds__(kTmThreads, 1) k_spread_tm(const float2* __res
     const int eL = 32 * q + lane, ea = eL / E1, ep1 = eL - ea * E1;
     float* const stg = reinterpret_cast<float*>(smem + L.stg_off) + eL * kTmStgStride;  // + 128 mt rows
     uint32_t k = 0;
-    int4 nxt = (int)blockIdx.x < num_items ? bins.items[blockIdx.x] : make_int4(0, 0, 0, 0);
-    for (int it = blockIdx.x; it < num_items; it += G, ++k) {
+    int4 nxt = tm_item(bins, blockIdx.x, num_items);
+    for (int it = blockIdx.x; it < num_items; it = tm_next_item(it), ++k) {
       const int4 item = nxt;
-      if (it + G < num_items) nxt = bins.items[it + G];  // one item ahead
+      nxt = tm_item(bins, tm_next_item(it), num_items);  // one item ahead
       tc::bulk_wait_read();  // the previous item's reductions have read the staging rows
       for (int mt = 0; mt < L.mt && healthy; ++mt) {
         healthy = __all_sync(0xffffffffu, tc::mbar_wait_bounded(&acc_full[mt], k & 1u, kTcPolls));
