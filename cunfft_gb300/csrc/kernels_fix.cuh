@@ -43,7 +43,8 @@ constexpr int kFixExpLo = 100, kFixExpHi = 1900;  // biased exponents the fixed-
 __host__ __device__ constexpr int fix_interp_warps(int d) { return d == 3 ? 16 : 8; }
 __host__ __device__ constexpr int fix_nodes_per_warp(int d) { return d == 1 ? 32 : (d == 3 ? 2 : 8); }
 __host__ __device__ constexpr int fix_spread_warps(int d) { return d == 3 ? 16 : (d == 2 ? 8 : 4); }
-__host__ __device__ constexpr int fix_batch(int d) { return d == 3 ? 20 : 64; }
+// d = 3 in slabs: 40 nodes between barriers where they leave room for kFixSlabPlanes planes
+__host__ __device__ constexpr int fix_batch(int d, int W) { return d == 3 ? (W > 14 && W <= 26 ? 40 : 20) : 64; }
 // CTAs per SM the registers are limited for: in 1D and 2D an item is a few short phases
 // between barriers, which other CTAs fill (2D, m = 6, M = 2^18: spreading 252 -> 223 us,
 // interpolation 149 -> 140 us)
@@ -55,7 +56,10 @@ __host__ __device__ constexpr int fix_spread_groups(int W) { return W <= 16 ? 2 
 // d = 3: up to this many taps the whole padded tile of 8 window starts fits in shared
 // memory; wider windows go through it in slabs of planes
 constexpr int kFixWholeW = 14;
-// d = 3 spreading in slabs: planes per slab, one for each pair of warps
+// d = 3 spreading in slabs: planes per slab, one for each pair of warps.  Full slabs and a
+// short last one: 33 planes (W = 26) as 8 + 8 + 8 + 8 + 1 instead of five of 7, where two of the
+// 16 warps idle.  With 40 nodes per batch: n = 128^3, M = 2^18 adjoint, W = 18 6.49 -> 6.06 ms,
+// W = 20 7.05 -> 6.54, W = 26 11.12 -> 10.24, W = 32 (no change) 14.75.
 constexpr int kFixSlabPlanes = 8;
 
 // Shared memory beyond the tile.
@@ -65,7 +69,7 @@ __host__ __device__ constexpr size_t fix_extra_smem(int d, int W, bool spread) {
   // are known), node and window start
   if (!spread) return tab + (size_t)fix_interp_warps(d) * fix_nodes_per_warp(d) * (d * W * sizeof(int2) + 2 * sizeof(int));
   // spreading, per node: taps, (P, Q), sample, sample x last-dimension taps, window start
-  return tab + (size_t)fix_batch(d) * (d * W * sizeof(int2) + d * sizeof(FixGauss) + sizeof(int4) +
+  return tab + (size_t)fix_batch(d, W) * (d * W * sizeof(int2) + d * sizeof(FixGauss) + sizeof(int4) +
                                        (d > 1 ? W * sizeof(int4) : 0) + sizeof(int));
 }
 
@@ -470,7 +474,7 @@ template <int D, int W, bool SLAB>
 __global__ void __launch_bounds__(fix_spread_warps(D) * 32, fix_ctas(D, W, true))
     k_spread_fix(const double2* __restrict__ f, double2* __restrict__ g, Geom geo, Tiling tl, Bins bins, FixPar fp) {
   constexpr int R = kWarp / W;
-  constexpr int NBC = fix_batch(D), NW = fix_spread_warps(D);
+  constexpr int NBC = fix_batch(D, W), NW = fix_spread_warps(D);
   constexpr int NP = D == 3 ? 2 : 1;  // d = 3: two warps share a row group, by plane parity
   constexpr int NG = NW / NP;
   constexpr int SH = off_bits(D);
