@@ -116,6 +116,10 @@ __host__ __device__ constexpr int fixed_plane_stride(int d, int W) {
   return d == 3 ? (fixed_t_mid(d, W) + W - 1) * fixed_row_stride(d, W) : fixed_row_stride(d, W);
 }
 
+// FP32 windows whose padded tile of a single plane of window starts does not fit in shared memory
+// go through it in slabs of planes
+__host__ __device__ constexpr bool grid_slabs(int d, int W) { return d == 3 && W > 24; }
+
 // The FP64 form's tiles (kernels_fix.cuh): 8 x 16 inner window starts in 3D for every W,
 // since tiles too large for shared memory go through it in slabs of planes.
 __host__ __device__ constexpr int fix_t_last(int d) { return d == 3 ? 16 : (d == 2 ? 64 : 1); }
@@ -148,9 +152,9 @@ struct Tiling {
   int chunk;             // max nodes per work item
   int threads;           // CTA size of the gridding kernels
   size_t smem_tile;      // bytes of the staged tile
-  int use_global;        // 1: no shared-memory tile fits, grid in global memory
-  int spread_kernel;     // spreading kernel in use: CUNFFT_X_SPREAD_SHARED, _REGISTER, _TENSOR or _GLOBAL
-  int interp_kernel;     // interpolation kernel in use: CUNFFT_X_INTERP_SHARED, _TENSOR or _GLOBAL
+  int slab;              // planes of the padded tile in shared memory at a time (E[0]: all of them)
+  int spread_kernel;     // spreading kernel in use: CUNFFT_X_SPREAD_SHARED, _REGISTER or _TENSOR
+  int interp_kernel;     // interpolation kernel in use: CUNFFT_X_INTERP_SHARED or _TENSOR
   // Sub-bins (sub_on = 1): the counting sort orders the nodes of a tile by sub-bin of
   // 2^ssh[0] x 2^ssh[1] window starts (dimensions 0 and 1), sub-bin (s0, s1) = s0 snb1 + s1
   // of ns per tile.  2D FP32 plans the tensor-core interpolation covers take 16 x 16

@@ -56,10 +56,7 @@ size_t gridding_smem_bytes(const Plan& p) {
   return p.tl.smem_tile + (a > b ? a : b);
 }
 
-cudaError_t grid_launch_global(const Plan&, bool, const void*, void*, cudaStream_t);
-
 static cudaError_t dispatch(const Plan& p, bool spread, const void* in, void* out, cudaStream_t st) {
-  if (p.tl.use_global) return grid_launch_global(p, spread, in, out, st);
   if (spread && p.tl.spread_kernel == CUNFFT_X_SPREAD_TENSOR) return grid_launch_spread_tc(p, in, out, st);
   if (!spread && p.tl.interp_kernel == CUNFFT_X_INTERP_TENSOR) return grid_launch_interp_tc(p, in, out, st);
   if (spread && p.tl.spread_kernel == CUNFFT_X_SPREAD_REGISTER) return grid_launch_spread_reg(p, in, out, st);

@@ -22,7 +22,7 @@ void interp2_tc_subbins(const Plan& p, Tiling& tl) {
   tl.ns = 1;
   tl.ssh[0] = tl.ssh[1] = 0;
   tl.snb1 = 1;
-  if (p.prec != kF32 || tl.use_global || !interp2_tc_ok(p.geo.d, p.geo.W, tl.T[1], p.geo.n[1])) return;
+  if (p.prec != kF32 || !interp2_tc_ok(p.geo.d, p.geo.W, tl.T[1], p.geo.n[1])) return;
   const int s0 = std::min(tl.T[0], kI2Sub);
   const int ns = (tl.T[0] / s0) * (tl.T[1] / kI2Sub);
   if (tl.tiles_total * ns >= ((int64_t)1 << 31)) return;  // sort keys are 32-bit
@@ -35,7 +35,7 @@ void interp2_tc_subbins(const Plan& p, Tiling& tl) {
 }
 
 bool interp2_tc_supported(const Plan& p) {
-  return p.geo.d == 2 && p.prec == kF32 && !p.tl.use_global && p.tl.sub_on && p.tl.sub_items;
+  return p.geo.d == 2 && p.prec == kF32 && p.tl.sub_on && p.tl.sub_items;
 }
 
 // Split rows half [batch][4][P0][P2s], row scales float [batch][P0], and the 5-D map over

@@ -16,7 +16,7 @@ cudaError_t grid_launch_interp2_tc(const Plan& p, const void* in, void* out, cud
 
 bool interp_tc_supported(const Plan& p) {
   if (p.geo.d == 2) return interp2_tc_supported(p);
-  return p.prec == kF32 && !p.tl.use_global && interp_tc_ok(p.geo.d, p.geo.W, p.tl.T[0], p.geo.n[2]);
+  return p.prec == kF32 && interp_tc_ok(p.geo.d, p.geo.W, p.tl.T[0], p.geo.n[2]);
 }
 
 // cuTensorMapEncodeTiled from the driver, through the runtime's entry-point query

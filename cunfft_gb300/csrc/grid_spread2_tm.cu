@@ -8,7 +8,7 @@
 namespace cg {
 
 bool spread2_tm_supported(const Plan& p) {
-  return p.prec == kF32 && !p.tl.use_global && spread2_tm_ok(p.geo.d, p.geo.W, p.tl.T[0], p.tl.T[1]);
+  return p.prec == kF32 && spread2_tm_ok(p.geo.d, p.geo.W, p.tl.T[0], p.tl.T[1]);
 }
 
 // The kernel allocates all 512 tensor-memory columns; its dynamic shared memory is at

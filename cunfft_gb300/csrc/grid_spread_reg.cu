@@ -33,7 +33,7 @@ size_t spread_reg_smem_bytes(const Plan& p) {
 }
 
 bool spread_reg_supported(const Plan& p) {
-  return p.prec == kF32 && !p.tl.use_global && spread_reg_ok(p.geo.d, p.geo.W, p.tl.T[0]);
+  return p.prec == kF32 && spread_reg_ok(p.geo.d, p.geo.W, p.tl.T[0]);
 }
 
 cudaError_t grid_launch_spread_reg(const Plan& p, const void* in, void* out, cudaStream_t st) {

@@ -6,7 +6,7 @@
 namespace cg {
 
 bool spread_tc_supported(const Plan& p) {
-  return (p.prec == kF32 && !p.tl.use_global && spread_tc_ok(p.geo.d, p.geo.W, p.tl.T[0])) ||
+  return (p.prec == kF32 && spread_tc_ok(p.geo.d, p.geo.W, p.tl.T[0])) ||
          spread2_tm_supported(p);
 }
 

@@ -7,7 +7,7 @@
 namespace cg {
 
 bool spread_tm_supported(const Plan& p) {
-  return p.prec == kF32 && !p.tl.use_global && spread_tm_ok(p.geo.d, p.geo.W, p.tl.T[0], p.tl.E[0]);
+  return p.prec == kF32 && spread_tm_ok(p.geo.d, p.geo.W, p.tl.T[0], p.tl.E[0]);
 }
 
 // The kernel allocates all 512 tensor-memory columns; its dynamic shared memory is at

@@ -129,7 +129,7 @@ static cudaError_t launch_grad_tile(const Plan& p, const void* g, const void* gr
 cudaError_t launch_interp_grad(const Plan& p, const void* g, const void* grad_f, double* grad_x, cudaStream_t st) {
   if (p.M == 0) return cudaSuccess;
   // the shared-tile kernels' shared memory covers the tile and more than the exponential's table
-  if (p.prec == kF32 && !p.tl.use_global) return launch_grad_tile(p, g, grad_f, grad_x, st);
+  if (p.prec == kF32 && p.tl.slab >= p.tl.E[0]) return launch_grad_tile(p, g, grad_f, grad_x, st);
   int64_t b = (p.M + 127) / 128;
   if (b > (int64_t)p.num_sms * 16) b = (int64_t)p.num_sms * 16;
   if (p.prec == kF64)

@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(kGradThreads)
   while (next_item(bins, 0, &cur)) {
     const int4 item = cur;
     const TileOrigin o = decode_tile<D>(geo, tl, item.x);
-    load_tile<D, W, float2>(tile, g + o.inst * geo.ntot, geo, tl, o);
+    load_tile<D, W, float2>(tile, g + o.inst * geo.ntot, geo, tl, o, 0, tl.E[0]);
     __syncthreads();
     for (int k = item.y + threadIdx.x; k < item.z; k += kGradThreads) {
       const int j = bins.sidx[k];

@@ -33,6 +33,13 @@
 //    the tile.  Batches are double-buffered (one barrier per batch).  The tile is
 //    then added to the global grid with vector atomics, so neighbouring items'
 //    halos combine.
+//  * Wide windows in 3D: above 16 taps a warp's lanes take consecutive cells of a plane's
+//    W x W window (interpolation; one row of W taps per pass left 32 - W lanes idle), and
+//    above 24 taps, where the padded tile of a single plane of window starts does not fit
+//    in shared memory, the tile goes through it in slabs of planes, interpolation adding
+//    each slab's part of a node.  n = 128^3, M = 2^18, interpolation with roll-off and FFT:
+//    W = 18 1.45 -> 0.99 ms, W = 22 2.08 -> 1.46; W = 26 17.0 -> 2.24 and spreading 20.2 ->
+//    4.54 (one thread per node through global memory before).
 //  * Tap weights: one hardware exp2 per tap in the FP32 form; in the FP64 form the reference's
 //    fast-Gaussian-gridding recurrence (2 exp per node and dim, src/cunfft_kernel.cu:
 //    491-505), which keeps the scarce FP64 pipe on the taps.
@@ -198,7 +205,7 @@ __device__ __forceinline__ int64_t row_gbase(const Geom& geo, const TileOrigin& 
 
 template <int D, int W, typename C>
 __device__ __forceinline__ void load_tile(C* tile, const C* __restrict__ gi, const Geom& geo, const Tiling& tl,
-                                          const TileOrigin& o) {
+                                          const TileOrigin& o, int p_lo, int p_n) {
   constexpr int S = fixed_row_stride(D, W), PS = fixed_plane_stride(D, W);
   const int E_last = tl.E[D - 1];
   const int64_t n_last = geo.n[D - 1], a_last = o.a[D - 1];
@@ -210,7 +217,7 @@ __device__ __forceinline__ void load_tile(C* tile, const C* __restrict__ gi, con
   // A lane's columns are the same in every row, and a warp steps from row to row without
   // divisions: the staging was a third of the instructions of an item of some 80 nodes.
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int rows = tile_rows<D>(tl), E1 = tl.E[1];
+  const int rows = D == 3 ? p_n * tl.E[1] : tile_rows<D>(tl), E1 = tl.E[1];
   constexpr int NC = (fixed_t_last(D, W) + W - 1 + kWarp - 1) / kWarp;
   int64_t col[NC];
 #pragma unroll
@@ -220,7 +227,7 @@ __device__ __forceinline__ void load_tile(C* tile, const C* __restrict__ gi, con
   const int d0 = D == 3 ? nwarps / E1 : nwarps, d1 = D == 3 ? nwarps - d0 * E1 : 0;
 #pragma unroll 4
   for (int row = warp; row < rows; row += nwarps) {
-    const C* src = gi + row_gbase<D>(geo, o, p0, p1);
+    const C* src = gi + row_gbase<D>(geo, o, p0 + p_lo, p1);
     C* dst = tile + (D == 3 ? p0 * PS + p1 * S : p0 * S) + lane;
 #pragma unroll
     for (int c = 0; c < NC; ++c)
@@ -240,11 +247,11 @@ __device__ __forceinline__ void load_tile(C* tile, const C* __restrict__ gi, con
 // float4 atomic.
 template <int D, int W, typename C>
 __device__ __forceinline__ void flush_tile(const C* tile, C* __restrict__ gi, const Geom& geo, const Tiling& tl,
-                                           const TileOrigin& o) {
+                                           const TileOrigin& o, int p_lo, int p_n) {
   constexpr int S = fixed_row_stride(D, W), PS = fixed_plane_stride(D, W);
   const int E_last = tl.E[D - 1];
   const int64_t n_last = geo.n[D - 1], a_last = o.a[D - 1];
-  const int rows = tile_rows<D>(tl);
+  const int rows = D == 3 ? p_n * tl.E[1] : tile_rows<D>(tl);
   constexpr bool kF32 = sizeof(C) == 8;
   const int tid = threadIdx.x, nt = blockDim.x;
   const bool pairs_ok = kF32 && (n_last & 1) == 0 && (tl.T[D - 1] & 1) == 0 &&  // even tile origin and row length
@@ -256,7 +263,7 @@ __device__ __forceinline__ void flush_tile(const C* tile, C* __restrict__ gi, co
     int p0, p1;
     row_coords<D>(tl, row, &p0, &p1);
     const C* src = tile + (D == 3 ? p0 * PS + p1 * S : (D == 2 ? p0 * S : 0));
-    const int64_t gb = row_gbase<D>(geo, o, p0, p1);
+    const int64_t gb = row_gbase<D>(geo, o, p0 + p_lo, p1);
     if (pairs_ok) {
       const int p = 2 * k;
       const C v0 = src[p];
@@ -304,7 +311,7 @@ __host__ __device__ inline size_t grid_extra_smem(int d, int W, size_t real, int
 // Interpolation, d = 1..3
 // ---------------------------------------------------------------------------
 template <int D, int W, typename T>
-__global__ void __launch_bounds__(512) k_interp(const typename Cx<T>::t* __restrict__ g,
+__global__ void __launch_bounds__(D == 3 && W > 16 ? 256 : 512) k_interp(const typename Cx<T>::t* __restrict__ g,
                                                 typename Cx<T>::t* __restrict__ f, Geom geo, Tiling tl, Bins bins) {
   using C = typename Cx<T>::t;
   constexpr int R = kWarp / W;           // rows (d >= 2) or nodes (d = 1) per warp pass
@@ -325,139 +332,177 @@ __global__ void __launch_bounds__(512) k_interp(const typename Cx<T>::t* __restr
   const T* sfrac = reinterpret_cast<const T*>(bins.sfrac);
   const T norm = (T)geo.norm;
   const int qd = lane / D, td = lane - qd * D;  // (node, dim) of this lane in the weight pass
+  // d = 3, W > 16: lane i takes cells i, i + 32, ... of a plane's W x W window, so that no lane
+  // idles where W does not divide 32 (bank i mod 16, as S == W mod 16)
+  constexpr bool FLAT = D == 3 && R == 1;
+  constexpr bool SLAB = grid_slabs(D, W);
+  constexpr int NF = FLAT ? (W * W + kWarp - 1) / kWarp : 1;
+  int fcell[NF];
+#pragma unroll
+  for (int i = 0; i < NF; ++i) {
+    const int c = min(lane + i * kWarp, W * W - 1);
+    fcell[i] = (c / W) * S + c % W;
+  }
 
   while (next_item(bins, 0, &cur)) {
     const int4 item = cur;
     const TileOrigin o = decode_tile<D>(geo, tl, item.x);
-    load_tile<D, W, C>(tile, g + o.inst * geo.ntot, geo, tl, o);
     // nodes per warp and batch: every warp has as many batches, as full as the next one's
     const int per = (item.z - item.y + nwarps - 1) / nwarps, nbat = (per + NB - 1) / NB;
     const int nbw = (per + nbat - 1) / nbat;
-    // records of this warp's first batch
-    int bs = item.y + warp * nbw;
-    int pf_idx = 0, pf_off = 0;
-    T pf_fr = 0;
-    if (bs < item.z) {
-      const int nb0 = min(nbw, item.z - bs);
-      if (lane < nb0) {
-        pf_idx = bins.sidx[bs + lane];
-        pf_off = bins.soff[bs + lane];
-      }
-      if (qd < nb0) pf_fr = sfrac[(int64_t)(bs + qd) * D + td];
-    }
-    __syncthreads();
-    for (; bs < item.z; bs += nwarps * nbw) {
-      const int nb = min(nbw, item.z - bs);
-      if (lane < nb) {
-        nrec[lane] = pf_idx;
-        nrec[NB + lane] = pf_off;
-      }
-      for (int qt0 = 0; qt0 < nb * D; qt0 += R) {
-        const int qt = qt0 + r;
-        const float fr = __shfl_sync(0xffffffffu, pf_fr, min(qt, 31));
-        if (lane_on && qt < nb * D) wb[qt * W + l_last] = WeightMath<T>::tap(fr + (float)(geo.m - l_last), geo, qt % D);
-      }
-      // fetch the next batch's records while this batch runs
-      const int bn = bs + nwarps * nbw;
-      if (bn < item.z) {
-        const int nbn = min(nbw, item.z - bn);
-        if (lane < nbn) {
-          pf_idx = bins.sidx[bn + lane];
-          pf_off = bins.soff[bn + lane];
+    for (int p_lo = 0; p_lo < (SLAB ? tl.E[0] : 1); p_lo += SLAB ? tl.slab : 1) {
+      const int p_n = SLAB ? min(tl.slab, tl.E[0] - p_lo) : tl.E[0];
+      load_tile<D, W, C>(tile, g + o.inst * geo.ntot, geo, tl, o, p_lo, p_n);
+      // records of this warp's first batch
+      int bs = item.y + warp * nbw;
+      int pf_idx = 0, pf_off = 0;
+      T pf_fr = 0;
+      if (bs < item.z) {
+        const int nb0 = min(nbw, item.z - bs);
+        if (lane < nb0) {
+          pf_idx = bins.sidx[bs + lane];
+          pf_off = bins.soff[bs + lane];
         }
-        if (qd < nbn) pf_fr = sfrac[(int64_t)(bn + qd) * D + td];
+        if (qd < nb0) pf_fr = sfrac[(int64_t)(bs + qd) * D + td];
       }
-      __syncwarp();
-      if (D == 1) {
-        for (int q0 = 0; q0 < nb; q0 += R) {
-          const int q = q0 + r;
-          const bool on = lane_on && q < nb;
-          const int qq = on ? q : q0;
-          const int o0 = nrec[NB + qq] & MASK;
-          C acc = on ? cscale(tile[o0 + l_last], wb[qq * W + l_last]) : czero<C>();
-#pragma unroll
-          for (int s = 1; s < W; s <<= 1) {
-            C o2;
-            o2.x = __shfl_down_sync(0xffffffffu, acc.x, s);
-            o2.y = __shfl_down_sync(0xffffffffu, acc.y, s);
-            if (l_last + s < W) {
-              acc.x += o2.x;
-              acc.y += o2.y;
-            }
+      __syncthreads();
+      for (; bs < item.z; bs += nwarps * nbw) {
+        const int nb = min(nbw, item.z - bs);
+        if (lane < nb) {
+          nrec[lane] = pf_idx;
+          nrec[NB + lane] = pf_off;
+        }
+        for (int qt0 = 0; qt0 < nb * D; qt0 += R) {
+          const int qt = qt0 + r;
+          const float fr = __shfl_sync(0xffffffffu, pf_fr, min(qt, 31));
+          if (lane_on && qt < nb * D) wb[qt * W + l_last] = WeightMath<T>::tap(fr + (float)(geo.m - l_last), geo, qt % D);
+        }
+        // fetch the next batch's records while this batch runs
+        const int bn = bs + nwarps * nbw;
+        if (bn < item.z) {
+          const int nbn = min(nbw, item.z - bn);
+          if (lane < nbn) {
+            pf_idx = bins.sidx[bn + lane];
+            pf_off = bins.soff[bn + lane];
           }
-          if (on && l_last == 0) f[nrec[qq]] = cscale(acc, norm);
+          if (qd < nbn) pf_fr = sfrac[(int64_t)(bn + qd) * D + td];
         }
-      } else {
-        // four nodes at a time: their lane sums are reduced together, each exchange halving
-        // what a lane holds (nodes, then components)
-        for (int q0 = 0; q0 < nb; q0 += 4) {
-          C accs[4];
+        __syncwarp();
+        if (D == 1) {
+          for (int q0 = 0; q0 < nb; q0 += R) {
+            const int q = q0 + r;
+            const bool on = lane_on && q < nb;
+            const int qq = on ? q : q0;
+            const int o0 = nrec[NB + qq] & MASK;
+            C acc = on ? cscale(tile[o0 + l_last], wb[qq * W + l_last]) : czero<C>();
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int q = q0 + u;
-            C acc = czero<C>();
-            if (q < nb && lane_on) {
-              const uint32_t off = (uint32_t)nrec[NB + q];
-              const T* wq = wb + q * D * W;
-              T wrow[NIT];
-#pragma unroll
-              for (int it = 0; it < NIT; ++it) {
-                const int lr = r + it * R;
-                wrow[it] = (FULL || lr < W) ? wq[(D - 2) * W + (FULL ? lr : min(lr, W - 1))] : (T)0;
+            for (int s = 1; s < W; s <<= 1) {
+              C o2;
+              o2.x = __shfl_down_sync(0xffffffffu, acc.x, s);
+              o2.y = __shfl_down_sync(0xffffffffu, acc.y, s);
+              if (l_last + s < W) {
+                acc.x += o2.x;
+                acc.y += o2.y;
               }
-              typename WPair<T>::t wpl[D == 3 ? W : 1];
-              if (D == 3) {
+            }
+            if (on && l_last == 0) f[nrec[qq]] = cscale(acc, norm);
+          }
+        } else {
+          // four nodes at a time: their lane sums are reduced together, each exchange halving
+          // what a lane holds (nodes, then components)
+          for (int q0 = 0; q0 < nb; q0 += 4) {
+            C accs[4];
 #pragma unroll
-                for (int l0 = 0; l0 < W; ++l0) wpl[l0] = WPair<T>::make(wq[l0]);
-              }
-              int base;
-              if (D == 3) {
+            for (int u = 0; u < 4; ++u) {
+              const int q = q0 + u;
+              C acc = czero<C>();
+              if (FLAT && q < nb) {
+                const uint32_t off = (uint32_t)nrec[NB + q];
+                const T* wq = wb + q * D * W;
                 const int o0 = off & MASK, o1 = (off >> SH) & MASK, o2 = off >> (D == 3 ? 2 * SH : 0);
-                base = o0 * PS + (o1 + r) * S + o2 + l_last;
-              } else {
-                const int o0 = off & MASK, o1 = (off >> SH) & MASK;
-                base = (o0 + r) * S + o1 + l_last;
-              }
-              const C* tb = tile + base;
+                const C* tb = tile + (o0 - p_lo) * PS + o1 * S + o2;
+                const int lo = SLAB ? max(0, p_lo - o0) : 0, hi = SLAB ? min(W, p_lo + p_n - o0) : W;  // planes of the slab
+                C ra[NF];
 #pragma unroll
-              for (int it = 0; it < NIT; ++it) {
-                if (FULL || r + it * R < W) {
-                  C ra;
-                  if (D == 3) {
-                    ra = czero<C>();
+                for (int i = 0; i < NF; ++i) ra[i] = czero<C>();
+#pragma unroll 2
+                for (int l0 = lo; l0 < hi; ++l0) {
+                  const typename WPair<T>::t w0 = WPair<T>::make(wq[l0]);
 #pragma unroll
-                    for (int l0 = 0; l0 < W; ++l0) ra = cmul_addp(ra, wpl[l0], tb[it * R * S + l0 * PS]);
-                  } else {
-                    ra = tb[it * R * S];
-                  }
-                  acc = cmul_add(acc, wrow[it], ra);
+                  for (int i = 0; i < NF; ++i) ra[i] = cmul_addp(ra[i], w0, tb[l0 * PS + fcell[i]]);
                 }
-              }
-              acc = cscale(acc, wq[(D - 1) * W + l_last]);
-            }
-            accs[u] = acc;
-          }
-          __syncwarp();
-          const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const C o2 = shfl_xor_c<C>(h16 ? accs[u] : accs[u + 2], 16);
-            const C a = h16 ? accs[u + 2] : accs[u];
-            accs[u].x = a.x + o2.x;
-            accs[u].y = a.y + o2.y;
+                for (int i = 0; i < NF; ++i) {
+                  const int c = min(lane + i * kWarp, W * W - 1);
+                  const T w12 = wq[(D - 2) * W + c / W] * wq[(D - 1) * W + c % W];
+                  if (i * kWarp + kWarp <= W * W || lane + i * kWarp < W * W) acc = cmul_add(acc, w12, ra[i]);
+                }
+              } else if (q < nb && lane_on) {
+                const uint32_t off = (uint32_t)nrec[NB + q];
+                const T* wq = wb + q * D * W;
+                T wrow[NIT];
+#pragma unroll
+                for (int it = 0; it < NIT; ++it) {
+                  const int lr = r + it * R;
+                  wrow[it] = (FULL || lr < W) ? wq[(D - 2) * W + (FULL ? lr : min(lr, W - 1))] : (T)0;
+                }
+                typename WPair<T>::t wpl[D == 3 ? W : 1];
+                if (D == 3) {
+#pragma unroll
+                  for (int l0 = 0; l0 < W; ++l0) wpl[l0] = WPair<T>::make(wq[l0]);
+                }
+                int base;
+                if (D == 3) {
+                  const int o0 = off & MASK, o1 = (off >> SH) & MASK, o2 = off >> (D == 3 ? 2 * SH : 0);
+                  base = o0 * PS + (o1 + r) * S + o2 + l_last;
+                } else {
+                  const int o0 = off & MASK, o1 = (off >> SH) & MASK;
+                  base = (o0 + r) * S + o1 + l_last;
+                }
+                const C* tb = tile + base;
+#pragma unroll
+                for (int it = 0; it < NIT; ++it) {
+                  if (FULL || r + it * R < W) {
+                    C ra;
+                    if (D == 3) {
+                      ra = czero<C>();
+#pragma unroll
+                      for (int l0 = 0; l0 < W; ++l0) ra = cmul_addp(ra, wpl[l0], tb[it * R * S + l0 * PS]);
+                    } else {
+                      ra = tb[it * R * S];
+                    }
+                    acc = cmul_add(acc, wrow[it], ra);
+                  }
+                }
+                acc = cscale(acc, wq[(D - 1) * W + l_last]);
+              }
+              accs[u] = acc;
+            }
+            __syncwarp();
+            const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const C o2 = shfl_xor_c<C>(h16 ? accs[u] : accs[u + 2], 16);
+              const C a = h16 ? accs[u + 2] : accs[u];
+              accs[u].x = a.x + o2.x;
+              accs[u].y = a.y + o2.y;
+            }
+            const C o2 = shfl_xor_c<C>(h8 ? accs[0] : accs[1], 8), a = h8 ? accs[1] : accs[0];
+            const T ax = a.x + o2.x, ay = a.y + o2.y;
+            T v = (h4 ? ay : ax) + __shfl_xor_sync(0xffffffffu, h4 ? ax : ay, 4);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            const int q = q0 + (h16 ? 2 : 0) + (h8 ? 1 : 0);
+            if ((lane & 3) == 0 && q < nb) {
+              T* dst = reinterpret_cast<T*>(f + nrec[q]) + (h4 ? 1 : 0);
+              *dst = SLAB && p_lo > 0 ? *dst + v * norm : v * norm;
+            }
           }
-          const C o2 = shfl_xor_c<C>(h8 ? accs[0] : accs[1], 8), a = h8 ? accs[1] : accs[0];
-          const T ax = a.x + o2.x, ay = a.y + o2.y;
-          T v = (h4 ? ay : ax) + __shfl_xor_sync(0xffffffffu, h4 ? ax : ay, 4);
-          v += __shfl_xor_sync(0xffffffffu, v, 2);
-          v += __shfl_xor_sync(0xffffffffu, v, 1);
-          const int q = q0 + (h16 ? 2 : 0) + (h8 ? 1 : 0);
-          if ((lane & 3) == 0 && q < nb) reinterpret_cast<T*>(f + nrec[q])[h4 ? 1 : 0] = v * norm;
         }
+        __syncwarp();
       }
-      __syncwarp();
+      __syncthreads();
     }
-    __syncthreads();
   }
 }
 
@@ -479,7 +524,8 @@ __global__ void __launch_bounds__(512) k_spread(const typename Cx<T>::t* __restr
   __shared__ int4 cur;
   C* tile = reinterpret_cast<C*>(smem);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int tile_elems = D == 1 ? tl.E[0] : (D == 2 ? tl.E[0] * S : tl.E[0] * PS);
+  constexpr bool SLAB = grid_slabs(D, W);
+  const int tile_elems = D == 1 ? tl.E[0] : (D == 2 ? tl.E[0] * S : tl.slab * PS);
   // d = 1: one private tile copy per warp (copy 0 is `tile`)
   const size_t extra = D == 1 ? (size_t)(nwarps - 1) * tl.smem_tile : 0;
   unsigned char* bptr = smem + tl.smem_tile + extra;
@@ -495,123 +541,127 @@ __global__ void __launch_bounds__(512) k_spread(const typename Cx<T>::t* __restr
   while (next_item(bins, 1, &cur)) {
     const int4 item = cur;
     const TileOrigin o = decode_tile<D>(geo, tl, item.x);
-    {
-      const C z = czero<C>();
-      if (D == 1) {
-        for (int e = lane; e < tile_elems; e += kWarp) mytile[e] = z;
-      } else {
-        for (int e = threadIdx.x; e < tile_elems; e += blockDim.x) tile[e] = z;
-      }
-    }
-    // records of the first batch
-    T pf_fr = 0;
-    int pf_off = 0;
-    C pf_val = czero<C>();
-    {
-      const int nb0 = min(NBC, item.z - item.y);
-      if (sq < nb0) pf_fr = sfrac[(int64_t)(item.y + sq) * D + st];
-      if ((int)threadIdx.x < nb0) {
-        pf_off = bins.soff[item.y + threadIdx.x];
-        pf_val = f[bins.sidx[item.y + threadIdx.x]];
-      }
-    }
-    int buf = 0;
-    for (int bs = item.y; bs < item.z; bs += NBC, buf ^= 1) {
-      const int nb = min(NBC, item.z - bs);
-      unsigned char* bb = bptr + buf * batch_bytes;
-      T* cw = reinterpret_cast<T*>(bb);                      // [NBC][D][W]
-      C* cval = reinterpret_cast<C*>(cw + NBC * D * W);      // [NBC]
-      int* coff = reinterpret_cast<int*>(cval + NBC);        // [NBC]
-      if (sq < nb) WeightMath<T>::taps(pf_fr, geo.m, geo, st, W, cw + (sq * D + st) * W);
-      if ((int)threadIdx.x < nb) {
-        coff[threadIdx.x] = pf_off;
-        cval[threadIdx.x] = cscale(pf_val, norm);
-      }
-      // fetch the next batch's records
-      const int bn = bs + NBC;
-      if (bn < item.z) {
-        const int nbn = min(NBC, item.z - bn);
-        if (sq < nbn) pf_fr = sfrac[(int64_t)(bn + sq) * D + st];
-        if ((int)threadIdx.x < nbn) {
-          pf_off = bins.soff[bn + threadIdx.x];
-          pf_val = f[bins.sidx[bn + threadIdx.x]];
+    for (int p_lo = 0; p_lo < (SLAB ? tl.E[0] : 1); p_lo += SLAB ? tl.slab : 1) {
+      const int p_n = SLAB ? min(tl.slab, tl.E[0] - p_lo) : tl.E[0];
+      {
+        const C z = czero<C>();
+        if (D == 1) {
+          for (int e = lane; e < tile_elems; e += kWarp) mytile[e] = z;
+        } else {
+          for (int e = threadIdx.x; e < tile_elems; e += blockDim.x) tile[e] = z;
         }
       }
-      __syncthreads();  // batch staged (and, for the first batch, the tile cleared)
-      if (D == 1) {
-        // warp w takes nodes w, w + nwarps, ...; lanes are the node's taps
-        for (int q = warp; q < nb; q += nwarps) {
-          const int o0 = coff[q] & MASK;
-          if (lane < W) {
-            C* p = mytile + o0 + lane;
-            *p = cmul_add(*p, cw[q * W + lane], cval[q]);
+      // records of the first batch
+      T pf_fr = 0;
+      int pf_off = 0;
+      C pf_val = czero<C>();
+      {
+        const int nb0 = min(NBC, item.z - item.y);
+        if (sq < nb0) pf_fr = sfrac[(int64_t)(item.y + sq) * D + st];
+        if ((int)threadIdx.x < nb0) {
+          pf_off = bins.soff[item.y + threadIdx.x];
+          pf_val = f[bins.sidx[item.y + threadIdx.x]];
+        }
+      }
+      int buf = 0;
+      for (int bs = item.y; bs < item.z; bs += NBC, buf ^= 1) {
+        const int nb = min(NBC, item.z - bs);
+        unsigned char* bb = bptr + buf * batch_bytes;
+        T* cw = reinterpret_cast<T*>(bb);                      // [NBC][D][W]
+        C* cval = reinterpret_cast<C*>(cw + NBC * D * W);      // [NBC]
+        int* coff = reinterpret_cast<int*>(cval + NBC);        // [NBC]
+        if (sq < nb) WeightMath<T>::taps(pf_fr, geo.m, geo, st, W, cw + (sq * D + st) * W);
+        if ((int)threadIdx.x < nb) {
+          coff[threadIdx.x] = pf_off;
+          cval[threadIdx.x] = cscale(pf_val, norm);
+        }
+        // fetch the next batch's records
+        const int bn = bs + NBC;
+        if (bn < item.z) {
+          const int nbn = min(NBC, item.z - bn);
+          if (sq < nbn) pf_fr = sfrac[(int64_t)(bn + sq) * D + st];
+          if ((int)threadIdx.x < nbn) {
+            pf_off = bins.soff[bn + threadIdx.x];
+            pf_val = f[bins.sidx[bn + threadIdx.x]];
           }
         }
-      } else if (D == 2) {
-        // warp w owns the row groups {g : g % nwarps == w}, group g = rows g*R .. g*R+R-1
-        for (int q = 0; q < nb; ++q) {
-          const uint32_t off = (uint32_t)coff[q];
-          const int o0 = off & MASK, o1 = (off >> SH) & MASK;
-          const int g_first = o0 / R, g_last = (o0 + W - 1) / R;
-          const int g0 = g_first + ((warp - g_first % nwarps) + nwarps) % nwarps;
-          if (g0 > g_last || !lane_on) continue;
-          const T* wq = cw + q * 2 * W;
-          const C v = cscale(cval[q], wq[W + l_last]);
-          C* tb = tile + o1 + l_last;
-          for (int gg = g0; gg <= g_last; gg += nwarps) {
-            const int p0 = gg * R + r;
-            if (p0 >= o0 && p0 < o0 + W) {
-              C* p = tb + p0 * S;
-              *p = cmul_add(*p, wq[p0 - o0], v);
+        __syncthreads();  // batch staged (and, for the first batch, the tile cleared)
+        if (D == 1) {
+          // warp w takes nodes w, w + nwarps, ...; lanes are the node's taps
+          for (int q = warp; q < nb; q += nwarps) {
+            const int o0 = coff[q] & MASK;
+            if (lane < W) {
+              C* p = mytile + o0 + lane;
+              *p = cmul_add(*p, cw[q * W + lane], cval[q]);
             }
           }
-        }
-      } else {
-        // warp w owns the planes {p : p % nwarps == w}
-        for (int q = 0; q < nb; ++q) {
-          const uint32_t off = (uint32_t)coff[q];
-          const int o0 = off & MASK, o1 = (off >> SH) & MASK, o2 = off >> (D == 3 ? 2 * SH : 0);
-          int p = o0 + ((warp - o0 % nwarps) + nwarps) % nwarps;
-          if (p >= o0 + W || !lane_on) continue;
-          const T* wq = cw + q * 3 * W;
-          const C v = cscale(cval[q], wq[2 * W + l_last]);
-          C vr[NIT];
-#pragma unroll
-          for (int it = 0; it < NIT; ++it) {
-            const int l1 = r + it * R;
-            vr[it] = cscale(v, (FULL || l1 < W) ? wq[W + (FULL ? l1 : min(l1, W - 1))] : (T)0);
+        } else if (D == 2) {
+          // warp w owns the row groups {g : g % nwarps == w}, group g = rows g*R .. g*R+R-1
+          for (int q = 0; q < nb; ++q) {
+            const uint32_t off = (uint32_t)coff[q];
+            const int o0 = off & MASK, o1 = (off >> SH) & MASK;
+            const int g_first = o0 / R, g_last = (o0 + W - 1) / R;
+            const int g0 = g_first + ((warp - g_first % nwarps) + nwarps) % nwarps;
+            if (g0 > g_last || !lane_on) continue;
+            const T* wq = cw + q * 2 * W;
+            const C v = cscale(cval[q], wq[W + l_last]);
+            C* tb = tile + o1 + l_last;
+            for (int gg = g0; gg <= g_last; gg += nwarps) {
+              const int p0 = gg * R + r;
+              if (p0 >= o0 && p0 < o0 + W) {
+                C* p = tb + p0 * S;
+                *p = cmul_add(*p, wq[p0 - o0], v);
+              }
+            }
           }
-          C* tb = tile + (o1 + r) * S + o2 + l_last;
-          for (; p < o0 + W; p += nwarps) {
-            const typename WPair<T>::t w0 = WPair<T>::make(wq[p - o0]);
-            C* tp = tb + p * PS;
+        } else {
+          // warp w owns the planes {p : p % nwarps == w}
+          for (int q = 0; q < nb; ++q) {
+            const uint32_t off = (uint32_t)coff[q];
+            const int o0 = off & MASK, o1 = (off >> SH) & MASK, o2 = off >> (D == 3 ? 2 * SH : 0);
+            const int p_first = SLAB ? max(o0, p_lo) : o0, p_end = SLAB ? min(o0 + W, p_lo + p_n) : o0 + W;
+            int p = p_first + ((warp - p_first % nwarps) + nwarps) % nwarps;
+            if (p >= p_end || !lane_on) continue;
+            const T* wq = cw + q * 3 * W;
+            const C v = cscale(cval[q], wq[2 * W + l_last]);
+            C vr[NIT];
 #pragma unroll
             for (int it = 0; it < NIT; ++it) {
-              if (FULL || r + it * R < W) {
-                C* t = tp + it * R * S;
-                *t = cmul_addp(*t, w0, vr[it]);
+              const int l1 = r + it * R;
+              vr[it] = cscale(v, (FULL || l1 < W) ? wq[W + (FULL ? l1 : min(l1, W - 1))] : (T)0);
+            }
+            C* tb = tile + (o1 + r) * S + o2 + l_last;
+            for (; p < p_end; p += nwarps) {
+              const typename WPair<T>::t w0 = WPair<T>::make(wq[p - o0]);
+              C* tp = tb + (p - p_lo) * PS;
+#pragma unroll
+              for (int it = 0; it < NIT; ++it) {
+                if (FULL || r + it * R < W) {
+                  C* t = tp + it * R * S;
+                  *t = cmul_addp(*t, w0, vr[it]);
+                }
               }
             }
           }
         }
       }
-    }
-    __syncthreads();
-    if (D == 1) {
-      // fold the private copies into copy 0, then flush
-      for (int e = threadIdx.x; e < tile_elems; e += blockDim.x) {
-        C s = tile[e];
-        for (int w = 1; w < nwarps; ++w) {
-          const C v = reinterpret_cast<const C*>(smem + (size_t)w * tl.smem_tile)[e];
-          s.x += v.x;
-          s.y += v.y;
+      __syncthreads();
+      if (D == 1) {
+        // fold the private copies into copy 0, then flush
+        for (int e = threadIdx.x; e < tile_elems; e += blockDim.x) {
+          C s = tile[e];
+          for (int w = 1; w < nwarps; ++w) {
+            const C v = reinterpret_cast<const C*>(smem + (size_t)w * tl.smem_tile)[e];
+            s.x += v.x;
+            s.y += v.y;
+          }
+          tile[e] = s;
         }
-        tile[e] = s;
+        __syncthreads();
       }
+      flush_tile<D, W, C>(tile, g + o.inst * geo.ntot, geo, tl, o, p_lo, p_n);
       __syncthreads();
     }
-    flush_tile<D, W, C>(tile, g + o.inst * geo.ntot, geo, tl, o);
-    __syncthreads();
   }
 }
 

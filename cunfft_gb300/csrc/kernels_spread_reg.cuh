@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(spread_reg_threads_max<W>()) k_spread_reg(cons
     }
     __syncthreads();
     const TileOrigin o = decode_tile<3>(geo, tl, item.x);
-    flush_tile<3, W, float2>(tile, g + o.inst * geo.ntot, geo, tl, o);
+    flush_tile<3, W, float2>(tile, g + o.inst * geo.ntot, geo, tl, o, 0, tl.E[0]);
     __syncthreads();  // every warp is done with `cur` and the batch buffers
   }
 }

@@ -166,7 +166,7 @@ static Tiling make_tiling(const Plan* p, const int* T, int chunk) {
   const bool t2 = d == 2 && p->prec == kF32 && W <= 16;
   // FP64 (fixed point): 512 nodes leave a cell's sum 53 bits below the largest sample
   tl.chunk = chunk > 0 ? chunk : (p->prec == kF64 ? 512 : (d == 3 ? 1024 : (t2 ? 256 : 2048)));
-  tl.use_global = 0;
+  tl.slab = tl.E[0];
   tl.ns = 1;  // no sub-bins unless the plan asks for them (plan_choose_tiling)
   return tl;
 }
@@ -179,7 +179,6 @@ static size_t smem_of(const Plan* p, const Tiling& tl) {
 
 // Spreading kernel for the plan's current tiling under a request (plan_set_spread_kernel).
 static int pick_spread_kernel(const Plan& p, int mode) {
-  if (p.tl.use_global) return CUNFFT_X_SPREAD_GLOBAL;
   const bool tc = spread_tc_supported(p), reg = spread_reg_supported(p);
   if (mode == CUNFFT_X_SPREAD_TENSOR) return tc ? CUNFFT_X_SPREAD_TENSOR : CUNFFT_X_SPREAD_SHARED;
   if (mode == CUNFFT_X_SPREAD_REGISTER) return reg ? CUNFFT_X_SPREAD_REGISTER : CUNFFT_X_SPREAD_SHARED;
@@ -189,15 +188,14 @@ static int pick_spread_kernel(const Plan& p, int mode) {
 
 // Interpolation kernel for the plan's current tiling under a request (plan_set_interp_kernel).
 static int pick_interp_kernel(const Plan& p, int mode) {
-  if (p.tl.use_global) return CUNFFT_X_INTERP_GLOBAL;
   if (mode == CUNFFT_X_INTERP_SHARED) return CUNFFT_X_INTERP_SHARED;
   return interp_tc_supported(p) ? CUNFFT_X_INTERP_TENSOR : CUNFFT_X_INTERP_SHARED;
 }
 
 // Tile extents: the caller's (or the defaults), clamped to the grid.  When the
 // padded tile does not fit in shared memory the largest extent is halved until it
-// does; when even 1-cell tiles do not fit (wide windows in 3D), the gridding runs
-// on the global-memory kernels with the default tiles as work items.
+// does; when even a single plane of window starts does not fit (3D, more than 24 taps),
+// the default tiles go through shared memory in equal slabs of planes, as few as fit.
 int plan_choose_tiling(Plan* p, const int* Tin, int chunk) {
   const int d = p->geo.d;
   const size_t kMaxSmem = 227 * 1024;
@@ -221,8 +219,12 @@ int plan_choose_tiling(Plan* p, const int* Tin, int chunk) {
     for (int t = 0; t < d; ++t)
       while (T[t] > p->geo.n[t]) T[t] >>= 1;
     tl = make_tiling(p, T, chunk);
-    tl.use_global = 1;
-    tl.threads = 128;
+    const size_t plane = tl.smem_tile / tl.E[0];
+    for (int parts = 2; smem_of(p, tl) > kMaxSmem && grid_slabs(d, p->geo.W) && tl.slab > 1; ++parts) {
+      tl.slab = (tl.E[0] + parts - 1) / parts;
+      tl.smem_tile = (plane * tl.slab + 15) / 16 * 16;
+    }
+    if (smem_of(p, tl) > kMaxSmem) return set_status(p, CUNFFT_X_UNSUPPORTED, "no tile fits in shared memory");
   }
   if (tl.tiles_total >= (int64_t)1 << 31) return set_status(p, CUNFFT_X_INVALID_ARGUMENT, "too many tiles");
   interp2_tc_subbins(*p, tl);
@@ -850,7 +852,7 @@ int plan_autotune(Plan* p, int reps) {
     if (p->spread_mode == CUNFFT_X_SPREAD_AUTO) {
       if (p->tl.spread_kernel != CUNFFT_X_SPREAD_REGISTER && spread_reg_supported(*p))
         skinds.push_back(CUNFFT_X_SPREAD_REGISTER);
-      if (p->tl.spread_kernel != CUNFFT_X_SPREAD_GLOBAL && p->tl.spread_kernel != CUNFFT_X_SPREAD_SHARED)
+      if (p->tl.spread_kernel != CUNFFT_X_SPREAD_SHARED)
         skinds.push_back(CUNFFT_X_SPREAD_SHARED);
     }
     if (p->interp_mode == CUNFFT_X_INTERP_AUTO && p->tl.interp_kernel == CUNFFT_X_INTERP_TENSOR)

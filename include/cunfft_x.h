@@ -31,24 +31,23 @@ enum { CUNFFT_X_F64 = 0, CUNFFT_X_F32 = 1 };
 /** Spreading (adjoint gridding) kernel.  AUTO picks TENSOR where it applies
  *  (FP32, 2m+2 <= 16, and d = 3 with outer tile extent <= 16 or d = 2 with tile
  *  extents <= 64), else REGISTER (d = 3, FP32, 2m+2 <= 16, outer tile extent <= 8),
- *  else SHARED; GLOBAL is reported when no shared-memory tile fits (wide 3D windows). */
+ *  else SHARED (the widest 3D windows in slabs of planes). */
 enum {
   CUNFFT_X_SPREAD_AUTO = 0,
   CUNFFT_X_SPREAD_SHARED = 1,   /* padded tile in shared memory, warp-owned planes */
   CUNFFT_X_SPREAD_REGISTER = 2, /* padded tile in registers, one warp per plane */
-  CUNFFT_X_SPREAD_GLOBAL = 3,   /* atomics straight into the grid (fallback) */
+  CUNFFT_X_SPREAD_GLOBAL = 3,   /* not reported any more: wide windows take SHARED in slabs of planes */
   CUNFFT_X_SPREAD_TENSOR = 4    /* tile update as FP16 hi/lo x3 tcgen05 MMAs, tile in tensor memory */
 };
 
 /** Interpolation (forward gridding) kernel.  AUTO picks TENSOR where it applies
  *  (FP32, 2m+2 <= 16; in 3D an outer tile extent <= 16 and n_3 divisible by 8; in 2D an
  *  inner tile extent >= 16 and n_2 divisible by 8, where the binning orders each tile's
- *  nodes by 16 x 16 sub-tile) and SHARED elsewhere; GLOBAL is reported when no
- *  shared-memory tile fits. */
+ *  nodes by 16 x 16 sub-tile) and SHARED elsewhere. */
 enum {
   CUNFFT_X_INTERP_AUTO = 0,
   CUNFFT_X_INTERP_SHARED = 1,   /* tile staged in shared memory, warp per node */
-  CUNFFT_X_INTERP_GLOBAL = 3,   /* taps read straight from the grid (fallback) */
+  CUNFFT_X_INTERP_GLOBAL = 3,   /* not reported any more: wide windows take SHARED in slabs of planes */
   CUNFFT_X_INTERP_TENSOR = 4    /* innermost contraction as FP16 hi/lo x3 tcgen05 MMAs */
 };
 
@@ -208,7 +207,7 @@ int cunfft_x_get_tiling(const cunfft_x_plan *plan, int *T, int *chunk, int *thre
  *  later tilings (a tiling the requested kernel does not cover runs SHARED). */
 int cunfft_x_set_spread_kernel(cunfft_x_plan *plan, int kind);
 
-/** Spreading kernel in use: CUNFFT_X_SPREAD_SHARED, _REGISTER, _TENSOR or _GLOBAL. */
+/** Spreading kernel in use: CUNFFT_X_SPREAD_SHARED, _REGISTER or _TENSOR. */
 int cunfft_x_get_spread_kernel(const cunfft_x_plan *plan, int *kind);
 
 /** Window of the gridding.  GAUSSIAN is the reference's (src/cunfft.cu:60-87: taps
@@ -236,7 +235,7 @@ int cunfft_x_get_window(const cunfft_x_plan *plan, int *window);
  *  holds across later tilings (a tiling TENSOR does not cover runs SHARED). */
 int cunfft_x_set_interp_kernel(cunfft_x_plan *plan, int kind);
 
-/** Interpolation kernel in use: CUNFFT_X_INTERP_SHARED, _TENSOR or _GLOBAL. */
+/** Interpolation kernel in use: CUNFFT_X_INTERP_SHARED or _TENSOR. */
 int cunfft_x_get_interp_kernel(const cunfft_x_plan *plan, int *kind);
 
 /** Per-stage device times of the last forward/adjoint call, in seconds
