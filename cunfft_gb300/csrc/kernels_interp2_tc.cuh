@@ -22,7 +22,7 @@
 // A sub-tile's B then is one TMA box (hi re, hi im, lo re, lo im; 32 halves x 32 rows each)
 // straight into the 64-byte swizzled K-major layout the MMAs read.
 //
-// Warp roles: two loader warps (warp 0 and the last one) issue the TMA loads and stage the
+// Warp roles: two loader warps issue the TMA loads and stage the
 // row scales, four warps issue the MMAs, two A sets of four warps build A and two reducing
 // sets of four warps sum the accumulators over each node's rows; every role takes the CTA's
 // items in turn.  Item li uses slot li % kI2Ring of A, B and the accumulators, so no warp
@@ -57,13 +57,13 @@ constexpr int kI2K = 32;                      // K: a sub-tile's 16 + W - 1 <= 3
 constexpr int kI2Rows = 32;                   // B rows per part: a sub-tile's 16 + W - 1 <= 31 rows, padded
 constexpr int kI2N = 2 * kI2Rows;             // MMA N: real parts 0..31, imaginary parts 32..63
 constexpr int kI2Sets = 2;                    // A-building sets and reducing sets, each on alternate items
+constexpr int kI2Loaders = 2;                 // TMA warps, each on every kI2Loaders-th item
 constexpr int kI2Issuers = 4;                 // MMA-issuing warps, each on every kI2Issuers-th item
-constexpr int kI2AWarp0 = 1 + kI2Issuers;     // two A sets of four warps
-constexpr int kI2RWarp0 = kI2AWarp0 + 4 * kI2Sets;  // two reducing sets of four warps
-constexpr int kI2Loaders = 2;                 // TMA warps, each on every kI2Loaders-th item: warp 0 and the last ones
-constexpr int kI2LWarp1 = kI2RWarp0 + 4 * kI2Sets;
-constexpr int kI2Threads = (kI2LWarp1 + kI2Loaders - 1) * 32;
+constexpr int kI2AWarp0 = kI2Loaders + kI2Issuers;  // warps 6-13: two A sets of four warps
+constexpr int kI2RWarp0 = kI2AWarp0 + 4 * kI2Sets;  // warps 14-21: two reducing sets of four warps
+constexpr int kI2Threads = (kI2RWarp0 + 4 * kI2Sets) * 32;
 constexpr int kI2Ring = 8;                    // slots of A, of B, and accumulators of kI2N columns (512 in all)
+constexpr int kI2ABufs = kI2Ring, kI2Stages = kI2Ring, kI2Acc = kI2Ring;
 constexpr int kI2Scales = 2 * kI2Ring;        // row-scale slots (item li's are read until its accumulator is)
 constexpr uint32_t kI2Part = kI2Rows * 64u;   // one B part (hi re, hi im, lo re, lo im): 32 rows x 64 bytes
 constexpr uint32_t kI2Stage = 4u * kI2Part;   // one slot of B, one TMA box: B hi = parts 0-1, B lo = parts 2-3
@@ -261,11 +261,11 @@ __global__ void __launch_bounds__(kI2Threads, 1) k_interp2_tc(const __grid_const
   // Item li of this CTA (li = 0, 1, ...) is bins.iitems[blockIdx.x + li G]; it uses slot
   // li % kI2Ring of every ring in its cycle li / kI2Ring, and A set and reducing set
   // li % kI2Sets.
-  if (warp == 0 || warp >= kI2LWarp1) {
+  if (warp < kI2Loaders) {
     // ======================= TMA: sub-tiles; their row scales =======================
     // The lanes decode 32 items at a time, one window ahead of their use.  Lane r loads the next item's row scale r and stores the current one's.
     const int64_t P0 = i2_split_dims(geo).P0;
-    const int ld = warp == 0 ? 0 : warp - kI2LWarp1 + 1;
+    const int ld = warp;
     auto load_key = [&](uint32_t first) {  // this warp's items first, first + 1, ...
       const int64_t i = (int64_t)blockIdx.x + ((int64_t)(first + lane) * kI2Loaders + ld) * G;
       return i < num_items ? bins.iitems[i].x : 0;
@@ -320,13 +320,13 @@ __global__ void __launch_bounds__(kI2Threads, 1) k_interp2_tc(const __grid_const
         healthy &= tc::mbar_wait_bounded(&bfull[(li - k) % kI2Ring], ((li - k) / kI2Ring) & 1u, kI2Polls);
     if (!healthy) *abort_flag = 1;
     __syncwarp();
-  } else if (warp <= kI2Issuers) {
+  } else if (warp < kI2AWarp0) {
     // ======================= MMA issuers: lane 0 =======================
     if (lane == 0) {
       const uint32_t sa = tc::smem_u32(smem + L.a_off), sb = tc::smem_u32(smem + L.b_off);
       const uint32_t idesc = tc::idesc_f16(128, kI2N);
-      uint32_t li = (uint32_t)(warp - 1);
-      for (int it = blockIdx.x + (warp - 1) * G; it < num_items; it += kI2Issuers * G, li += kI2Issuers) {
+      uint32_t li = (uint32_t)(warp - kI2Loaders);
+      for (int it = blockIdx.x + (warp - kI2Loaders) * G; it < num_items; it += kI2Issuers * G, li += kI2Issuers) {
         const uint32_t st = li % kI2Ring;
         bool ok = tc::mbar_wait_bounded(&afull[st], (li / kI2Ring) & 1u, kI2Polls);
         ok = ok && tc::mbar_wait_bounded(&bfull[st], (li / kI2Ring) & 1u, kI2Polls);
