@@ -552,7 +552,7 @@ def run_ours(args):
                                                                        fh_h_out.reshape(-1))}
     h2d = xh.numel() * 8 + fhh.numel() * 8 + fin_h.numel() * 8
     d2h = fout_h.numel() * 8 + fh_h_out.numel() * 8
-    launches_per_step = (4 + 2 + 2 + (1 if p32.spread_kernel() == "tensor" else 0)
+    launches_per_step = (3 + 2 + 2 + (1 if p32.spread_kernel() == "tensor" else 0)
                          + interp_prep_launches(p32))
     tiling = p32.tiling()
     p32.close()
