@@ -24,6 +24,10 @@ def _ptr(t):
 class NFFT:
     def __init__(self, N, n=None, m=6, precision="f64", batch=1, device=None, stream=None, window="gaussian"):
         self._host_refs = []  # host tensors in flight in host-buffer transforms
+        # The device tensors of the last forward and adjoint transform.  A plan on the default
+        # stream runs on a private one, which torch's allocator does not know: a block that the
+        # caller drops while the plan still writes it could go to another plan's next output.
+        self._live = {}
         self._lib = nat.lib()
         self.N = [int(v) for v in N]
         self.d = len(self.N)
@@ -100,6 +104,10 @@ class NFFT:
             raise ValueError("f has the wrong size")
         return f
 
+    def _keep(self, what, a, out):
+        # without the autograd graph of an input
+        self._live[what] = (a.detach() if a.grad_fn is not None else a, out.detach() if out.grad_fn is not None else out)
+
     def _coef_shape(self):
         return ([self.batch] if self.batch > 1 else []) + self.N
 
@@ -107,12 +115,14 @@ class NFFT:
         fhat = self._coef(fhat)
         f = out if out is not None else torch.empty(self.M, dtype=self.cdtype, device=self.device)
         nat.check(self._lib.cunfft_x_forward(self._h, _ptr(fhat), _ptr(f)), self._h)
+        self._keep("forward", fhat, f)
         return f
 
     def adjoint(self, f, out=None):
         f = self._samples(f)
         fh = out if out is not None else torch.empty(self._coef_shape(), dtype=self.cdtype, device=self.device)
         nat.check(self._lib.cunfft_x_adjoint(self._h, _ptr(f), _ptr(fh)), self._h)
+        self._keep("adjoint", f, fh)
         return fh
 
     # ------------------------------------------------ host buffers, overlapped copies
@@ -272,6 +282,7 @@ class NFFT:
     def synchronize(self):
         nat.check(self._lib.cunfft_x_synchronize(self._h), self._h)
         self._host_refs = []  # host buffers of finished host-buffer transforms
+        self._live.clear()
 
     def grid(self):
         """The plan's oversampled grid as a tensor view (batch, *n)."""
@@ -286,6 +297,7 @@ class NFFT:
         if getattr(self, "_h", None):
             self._lib.cunfft_x_plan_destroy(self._h)
             self._h = None
+            self._live.clear()
 
     def __del__(self):
         try:
