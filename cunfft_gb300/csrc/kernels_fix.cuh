@@ -25,7 +25,7 @@
 //
 // Measured against the FP64-pipe kernels before: 3D n = 128^3, M = 2^18, m = 6 interpolation
 // 4.18 -> 0.94 ms, spreading 5.75 -> 1.61 ms; m = 12 (global-memory kernels before)
-// 68.8 -> 5.9 and 43.2 -> 10.2 ms; 2D n = 1024^2, M = 2^18, m = 6 0.80 -> 0.16 and
+// 68.8 -> 5.9 and 43.2 -> 9.8 ms; 2D n = 1024^2, M = 2^18, m = 6 0.80 -> 0.16 and
 // 1.00 -> 0.28 ms.  Relative l2 error against 64-bit sums with exact taps: 4e-16 to 1.1e-15
 // for whole m = 6 transforms (4e-15 to 1.5e-14 before, from the recurrence taps).
 #pragma once
