@@ -2,8 +2,9 @@
 //
 // An FP64 FFT is bound by GB300's FP64 pipe (2 multiply-adds per clock and SM): the library's
 // 1024^2 transform takes 172 us, of which memory needs about 10.  Here a CTA transforms C
-// neighbouring lines of one dimension in shared memory with 64-bit integers (fixmath.h): the
-// loaded values are scaled by a power of two so that no sum can overflow, radix-4 passes
+// neighbouring lines of one dimension in shared memory with 64-bit integers (fixmath.h): each
+// line's values are scaled by a power of two of its own (neighbouring lines may belong to
+// different instances of a batch) so that no sum can overflow, radix-4 passes
 // (Stockham order: twiddle, butterfly, store; one radix-2 pass first when log2 L is odd) with
 // twiddles in units of 2^-62, whose product divides by four as the butterfly may multiply by
 // four, and FP64 again on the way out.  Rounding errors stay near 2^-54 of the lines' largest
@@ -32,6 +33,7 @@ namespace cg {
 
 constexpr int kFftThreads = 256;
 constexpr int kFftMaxL = 4096;  // points of a line in shared memory
+constexpr int kFftMaxC = 64;    // lines of a CTA, at most (16 points each)
 
 // One pass: FFTs along dimension t of the grid.
 struct FftArgs {
@@ -242,12 +244,12 @@ __device__ __forceinline__ void fft_run(double2 (&in)[TPT][4], unsigned char* sm
 template <int TPT, bool INV>
 __global__ void __launch_bounds__(kFftThreads, TPT == 4 ? 2 : 3) k_fft(FftArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ uint32_t s_top;
+  __shared__ uint32_t s_top[kFftMaxC];  // per line
   const int C = 1 << a.logC, L = 1 << a.logL, L4 = L >> 2;
   const int c = threadIdx.x & (C - 1), j0 = threadIdx.x >> a.logC, dj = kFftThreads >> a.logC;
   const uint32_t line = blockIdx.x * (uint32_t)C + c;
   const bool on = line < a.lines;
-  if (threadIdx.x == 0) s_top = 0;
+  if (threadIdx.x < C) s_top[threadIdx.x] = 0;
   // the line's place: (instance, leading indices) and tail
   const int64_t tail = (int64_t)1 << a.log_tail;
   const uint32_t tail_i = line & (uint32_t)(tail - 1);
@@ -303,11 +305,12 @@ __global__ void __launch_bounds__(kFftThreads, TPT == 4 ? 2 : 3) k_fft(FftArgs a
     }
   }
   __syncthreads();
-  top = __reduce_max_sync(0xffffffffu, top);
-  if ((threadIdx.x & 31) == 0) atomicMax(&s_top, top);
+  for (int o = 16; o >= C; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));  // the warp's lanes of a line
+  if ((threadIdx.x & 31) < C) atomicMax(&s_top[c], top);
   __syncthreads();
-  top = s_top;
+  top = s_top[c];
   const int key = fix_exp_of_hi(top);
+  const bool f64 = __syncthreads_or(top != 0 && (key < 100 || key > 1900));
   double2* out = a.dst + base;
   int64_t stride = tail;
   if (a.dst_l) {  // second 1D pass: line `lead` of instance `rest`, transposed
@@ -316,7 +319,7 @@ __global__ void __launch_bounds__(kFftThreads, TPT == 4 ? 2 : 3) k_fft(FftArgs a
   }
   // components below 2^58 (2^59 where the first pass only adds two): their complex values
   // times what the first pass adds stay below 2^61, the later passes keep that
-  if (top == 0 || (key >= 100 && key <= 1900))
+  if (!f64)
     fft_run<FftFix, TPT, INV>(in, smem, a, c, j0, dj, 58 + (a.logL & 1) - (key - 1022), on, tail_i, out, stride);
   else
     fft_run<FftF64, TPT, INV>(in, smem, a, c, j0, dj, 0, on, tail_i, out, stride);
