@@ -8,10 +8,12 @@
 // on the bits.
 //
 // Two products.  Interpolation adds many of them in registers and keeps the two orders
-// apart (FixSum).  A number v = v1 2^28 + v0 is a pair of limbs: weights have
-// -2^27 <= v0 < 2^27, values 0 <= v0 < 2^28;
+// apart (FixSum).  A number v = v1 2^28 + v0, -2^27 <= v0 < 2^27, is a pair of limbs;
 //   v w / 2^56 = v1 w1 + (v1 w0 + v0 w1) / 2^28 + v0 w0 / 2^56,
-// and the last term, at most half a unit of the result and zero on average, is left out.
+// and the last term, at most a quarter of a unit of the result, is left out.  It is zero on
+// average for every weight, as v0 is centred: with 0 <= v0 < 2^28 all cells of a plane shared
+// the offset w0 / 2^29, which the other two dimensions' weights add up while the values they
+// weigh cancel (3D, m = 12: relative error 4.8e-14 of an interpolation, 1.2e-14 centred).
 // Spreading adds one product at a time to a cell in shared memory (fix_mad62): limbs of 32
 // bits, v = v1 2^32 + v0 with -2^31 <= v0 < 2^31, weights in units of 2^-62, so that the
 // second order's shift is the choice of its high word:
@@ -38,20 +40,14 @@ struct FixPair {
   int32_t hi, lo;
 };
 
-// limbs of a weight: the low one centred
-CG_FIX_HD FixPair fix_split_w(int64_t v) {
+// limbs of a value, |v| < 2^59 - 2^27, and of a weight
+CG_FIX_HD FixPair fix_split(int64_t v) {
   FixPair p;
   p.lo = (int32_t)((uint32_t)v << (32 - kFixLimb)) >> (32 - kFixLimb);
   p.hi = (int32_t)((v - p.lo) >> kFixLimb);
   return p;
 }
-// limbs of a value: the low one non-negative
-CG_FIX_HD FixPair fix_split(int64_t v) {
-  FixPair p;
-  p.lo = (int32_t)((uint32_t)v & ((1u << kFixLimb) - 1u));
-  p.hi = (int32_t)(v >> kFixLimb);
-  return p;
-}
+CG_FIX_HD FixPair fix_split_w(int64_t v) { return fix_split(v); }
 
 // c + a b.  As a carry pair the two halves stay one multiply-add instruction; mad.wide the
 // assembler takes apart to shorten its chains, at the price of a 64-bit addition for every

@@ -13,8 +13,9 @@ CG_DECL(20) CG_DECL(22) CG_DECL(24) CG_DECL(26) CG_DECL(28) CG_DECL(30) CG_DECL(
 bool gridding_supported(int d, int W) { return d >= 1 && d <= 3 && W >= 4 && W <= 32 && (W % 2) == 0; }
 
 // Constants of the fixed-point gridding.  vbits: a node's sum is at most 2^vbits times the
-// product of the largest tap sums S_t per dimension, which has to stay below 2^62, and each
-// sum before the last dimension below 2^58, where its high limb still has 31 bits.
+// product of the largest tap sums S_t per dimension, which has to stay below 2^63, and each
+// sum before the last dimension below 2^59, where its high limb still fits 32 bits with its
+// sign (S_t is taken 2 % too large).
 FixPar fix_params(const Geom& g) {
   FixPar fp{};
   double all = 0.0, last = 0.0;
@@ -35,7 +36,7 @@ FixPar fix_params(const Geom& g) {
     last = log2(1.02 * most);  // between the sampled fractions the sum hardly moves
     all += last;
   }
-  const int a = (int)floor(62.0 - all), b = (int)floor(58.0 - (all - last));
+  const int a = (int)floor(63.0 - all), b = (int)floor(59.0 - (all - last));
   fp.vbits = a < b ? a : b;
   if (fp.vbits > 55) fp.vbits = 55;
   return fp;
