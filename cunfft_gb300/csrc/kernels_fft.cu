@@ -7,8 +7,10 @@
 // different instances of a batch) so that no sum can overflow, radix-4 passes
 // (Stockham order: twiddle, butterfly, store; one radix-2 pass first when log2 L is odd) with
 // twiddles in units of 2^-62, whose product divides by four as the butterfly may multiply by
-// four, and FP64 again on the way out.  Rounding errors stay near 2^-54 of the lines' largest
-// value per output, below an FP64 FFT's.  Lines whose values are not finite, or near FP64's
+// four, and FP64 again on the way out.  Where the sum of a line's magnitudes rules that growth
+// out, its values are shifted up first, so that a line of few large values keeps its bits too.
+// A pass's rounding errors stay below 2^-59 of the bound on its values, for dense lines 2^-54
+// of the result.  Lines whose values are not finite, or near FP64's
 // exponent limits, take the same passes in FP64.
 //
 // The forward transform is fused with the roll-off and skips the zero padding: a pass reads
@@ -20,8 +22,9 @@
 //
 // Bound: integer multiply-adds (9 per point and radix-4 pass at 29 per clock and SM) and the
 // 64-bit additions beside them.  Measured, forward with roll-off and
-// adjoint: 1024^2 46 and 46 us (library and roll-off kernel: 180 and 173), 128^3 56 and 88 us
-// (368 and 356), 2^18 22 and 21 us (96 and 92).
+// adjoint: 1024^2 51 and 54 us (library and roll-off kernel: 180 and 173), 128^3 68 and 101 us
+// (368 and 356), 2^18 29 and 27 us (96 and 92).  A scale and a sum per
+// line cost 5 to 10 % of that (1024^2 49 and 52 us, 128^3 63 and 89 with one scale per CTA).
 #include <math.h>
 
 #include <vector>
@@ -93,6 +96,12 @@ struct FftFix {
     return r;
   }
   static __device__ __forceinline__ double2 back(V v, int sc) { return make_double2(fix_to_f64(v.x, sc), fix_to_f64(v.y, sc)); }
+  static __device__ __forceinline__ V up(V v, int s) {
+    I2 r;
+    r.x = (int64_t)((uint64_t)v.x << s);
+    r.y = (int64_t)((uint64_t)v.y << s);
+    return r;
+  }
   static __device__ __forceinline__ V mul(V v, int4 w) { return fft_mul(v, w); }
   static __device__ __forceinline__ V quarter(V v) {
     I2 r;
@@ -110,6 +119,7 @@ struct FftF64 {
     const double hi = 4294967296.0;
     return make_double2(((double)w.x * hi + (double)w.y) * u, ((double)w.z * hi + (double)w.w) * u);
   }
+  static __device__ __forceinline__ V up(V v, int) { return v; }
   static __device__ __forceinline__ V mul(V v, int4 w) {
     const double2 t = tw(w);
     return make_double2(v.x * t.x - v.y * t.y, v.x * t.y + v.y * t.x);
@@ -156,9 +166,22 @@ __device__ __forceinline__ int4 fft_tw(const int4* __restrict__ t, int k, bool i
   return w;
 }
 
-// The passes over a CTA's lines: v holds, per task u, the points j + r L / 4 of line c.
+// Room of a line in fixed point: its complex values are below 2^(60.5 - room), and the passes
+// to come multiply them by 2^grow at most.
+struct FftRoom {
+  int room, grow;
+  __device__ __forceinline__ void pass(int g) {  // a pass that adds 2^g values
+    g = min(g, grow);
+    room -= g;
+    grow -= g;
+  }
+};
+
+// The passes over a CTA's lines: v holds, per task u, the points j + r L / 4 of line c.  Returns
+// the bits that the divisions took off the scale.
 template <typename A, int TPT, bool INV>
-__device__ __forceinline__ void fft_passes(typename A::V (&v)[TPT][4], typename A::V* buf, const FftArgs& a, int c, int j0, int dj) {
+__device__ __forceinline__ int fft_passes(typename A::V (&v)[TPT][4], typename A::V* buf, const FftArgs& a, int c, int j0, int dj,
+                                          FftRoom& rm) {
   using V = typename A::V;
   const int L4 = 1 << (a.logL - 2), lc = a.logC;
   int ns;
@@ -175,6 +198,7 @@ __device__ __forceinline__ void fft_passes(typename A::V (&v)[TPT][4], typename 
       buf[((2 * (j + L4) + 1) << lc) + c] = o1;
     }
     ns = 2;
+    rm.pass(1);
   } else {
 #pragma unroll
     for (int u = 0; u < TPT; ++u) {
@@ -184,8 +208,9 @@ __device__ __forceinline__ void fft_passes(typename A::V (&v)[TPT][4], typename 
       for (int r = 0; r < 4; ++r) buf[((4 * j + r) << lc) + c] = v[u][r];
     }
     ns = 4;
+    rm.pass(2);
   }
-  for (;; ns *= 4) {
+  for (int off = 0;; ns *= 4) {
     __syncthreads();
     const int step = L4 / ns;  // L / (4 ns)
 #pragma unroll
@@ -193,12 +218,15 @@ __device__ __forceinline__ void fft_passes(typename A::V (&v)[TPT][4], typename 
       const int j = j0 + u * dj, k = (j & (ns - 1)) * step;
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        const V t = buf[((j + r * L4) << lc) + c];
+        const V t = A::up(buf[((j + r * L4) << lc) + c], rm.room);
         v[u][r] = r == 0 ? A::quarter(t) : A::mul(t, fft_tw(a.tw, r * k, INV));
       }
       fft4<INV>(v[u]);
     }
-    if (ns == L4) return;  // the last pass: results at j + r L / 4
+    off += 2 - rm.room;
+    rm.room = 2;
+    rm.pass(2);
+    if (ns == L4) return off;  // the last pass: results at j + r L / 4
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < TPT; ++u) {
@@ -211,16 +239,14 @@ __device__ __forceinline__ void fft_passes(typename A::V (&v)[TPT][4], typename 
 
 template <typename A, int TPT, bool INV>
 __device__ __forceinline__ void fft_run(double2 (&in)[TPT][4], unsigned char* smem, const FftArgs& a, int c, int j0, int dj,
-                                        int sc, bool on, uint32_t tail_i, double2* out, int64_t stride) {
+                                        int sc, FftRoom rm, bool on, uint32_t tail_i, double2* out, int64_t stride) {
   using V = typename A::V;
   V v[TPT][4];
 #pragma unroll
   for (int u = 0; u < TPT; ++u)
 #pragma unroll
     for (int r = 0; r < 4; ++r) v[u][r] = A::make(in[u][r], sc);
-  fft_passes<A, TPT, INV>(v, reinterpret_cast<V*>(smem), a, c, j0, dj);
-  // every pass but the first divided by four (FP64: none), the post twiddle by four again
-  int so = sc - 2 * ((a.logL - 1) / 2);
+  const int so = sc - fft_passes<A, TPT, INV>(v, reinterpret_cast<V*>(smem), a, c, j0, dj, rm);  // (FP64: not used)
   const int L4 = 1 << (a.logL - 2);
   if (!on) return;
 #pragma unroll
@@ -232,24 +258,34 @@ __device__ __forceinline__ void fft_run(double2 (&in)[TPT][4], unsigned char* sm
       int s = so;
       if (a.post_hi) {
         const int64_t m = ((int64_t)l * tail_i) & (((int64_t)1 << a.post_log) - 1);
-        t = A::mul(A::mul(t, fft_tw(a.post_hi, (int)(m >> a.post_sh), INV)),
-                   fft_tw(a.post_lo, (int)(m & ((1 << a.post_sh) - 1)), INV));
-        s -= 4;
+        // two divisions by four; the first leaves room for two bits
+        t = A::mul(A::up(t, rm.room), fft_tw(a.post_hi, (int)(m >> a.post_sh), INV));
+        t = A::mul(A::up(t, 2), fft_tw(a.post_lo, (int)(m & ((1 << a.post_sh) - 1)), INV));
+        s -= 2 - rm.room;
       }
       out[l * stride] = A::back(t, s);
     }
   }
 }
 
+// |v| rounded up to a multiple of 2^(key - 1040); zero for zero and what the scale makes zero
+__device__ __forceinline__ uint32_t fft_mag(double v, int key) {
+  const uint32_t hi = (uint32_t)__double2hiint(v), e = fix_exp_of_hi(hi);
+  const uint32_t mant = (hi & 0xFFFFFu) | 0x100000u;  // 21 bits
+  return e == 0 ? 0u : (mant >> min(31u, 3u + (uint32_t)key - e)) + 1u;
+}
+
 template <int TPT, bool INV>
 __global__ void __launch_bounds__(kFftThreads, TPT == 4 ? 2 : 3) k_fft(FftArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ uint32_t s_top[kFftMaxC];  // per line
+  __shared__ uint32_t s_top[kFftMaxC], s_sum[kFftMaxC];  // per line
+  __shared__ int s_f64;
   const int C = 1 << a.logC, L = 1 << a.logL, L4 = L >> 2;
   const int c = threadIdx.x & (C - 1), j0 = threadIdx.x >> a.logC, dj = kFftThreads >> a.logC;
   const uint32_t line = blockIdx.x * (uint32_t)C + c;
   const bool on = line < a.lines;
-  if (threadIdx.x < C) s_top[threadIdx.x] = 0;
+  if (threadIdx.x < C) s_top[threadIdx.x] = s_sum[threadIdx.x] = 0;
+  if (threadIdx.x == 0) s_f64 = 0;
   // the line's place: (instance, leading indices) and tail
   const int64_t tail = (int64_t)1 << a.log_tail;
   const uint32_t tail_i = line & (uint32_t)(tail - 1);
@@ -310,19 +346,34 @@ __global__ void __launch_bounds__(kFftThreads, TPT == 4 ? 2 : 3) k_fft(FftArgs a
   __syncthreads();
   top = s_top[c];
   const int key = fix_exp_of_hi(top);
-  const bool f64 = __syncthreads_or(top != 0 && (key < 100 || key > 1900));
+  if (top != 0 && (key < 100 || key > 1900)) s_f64 = 1;
+  // sum of the components' magnitudes, rounded up, 2^18 standing for 2^(key - 1022) above the largest
+  uint32_t sum = 0;
+#pragma unroll
+  for (int u = 0; u < TPT; ++u)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) sum += fft_mag(in[u][r].x, key) + fft_mag(in[u][r].y, key);
+  for (int o = 16; o >= C; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) < C) atomicAdd(&s_sum[c], sum);
+  __syncthreads();
+  sum = s_sum[c];
+  const bool f64 = s_f64 != 0;
   double2* out = a.dst + base;
   int64_t stride = tail;
   if (a.dst_l) {  // second 1D pass: line `lead` of instance `rest`, transposed
     out = a.dst + rest * a.lead_n * L + lead;
     stride = a.dst_l;
   }
-  // components below 2^58 (2^59 where the first pass only adds two): their complex values
-  // times what the first pass adds stay below 2^61, the later passes keep that
+  // Components below 2^58 (2^59 where the first pass only adds two): with what the first pass
+  // adds, complex values stay below 2^60.5.  They never exceed the sum of the line's magnitudes,
+  // 2^grow times its largest: what a line of few large values does not grow, its divisions spare.
+  FftRoom rm;
+  rm.room = 2 - (a.logL & 1);
+  rm.grow = sum > (1u << 18) ? 14 - __clz(sum - 1) : 0;
   if (!f64)
-    fft_run<FftFix, TPT, INV>(in, smem, a, c, j0, dj, 58 + (a.logL & 1) - (key - 1022), on, tail_i, out, stride);
+    fft_run<FftFix, TPT, INV>(in, smem, a, c, j0, dj, 58 + (a.logL & 1) - (key - 1022), rm, on, tail_i, out, stride);
   else
-    fft_run<FftF64, TPT, INV>(in, smem, a, c, j0, dj, 0, on, tail_i, out, stride);
+    fft_run<FftF64, TPT, INV>(in, smem, a, c, j0, dj, 0, rm, on, tail_i, out, stride);
 }
 
 // ---------------------------------------------------------------------------
