@@ -131,6 +131,10 @@ __host__ __device__ constexpr int fix_plane_stride(int d, int W) {
   return d == 3 ? (fix_t_mid(d) + W - 1) * fix_row_stride(d, W) : fix_row_stride(d, W);
 }
 
+// The FP64 form's work items hold at most this many nodes, whatever the chunk: a spreading cell
+// leaves room for the sum of an item's samples, 2^9 of them at 53 bits below the largest.
+constexpr int kFixItem = 512;
+
 // Constants of the FP64 form's fixed-point gridding (kernels_fix.cuh), one set per plan.
 struct FixPar {
   uint64_t c60[kMaxDim];  // Gaussian: log2(e) / b_t in units of 2^-60 and of 2^-57
@@ -149,7 +153,8 @@ struct Tiling {
   int R1;                // rows per plane (E[d-2] for d = 3, unused otherwise)
   int64_t tiles_per_inst;
   int64_t tiles_total;   // batch * tiles_per_inst
-  int chunk;             // max nodes per work item
+  int chunk;             // max nodes per work item, as asked for
+  int item;              // max nodes per work item: chunk, in the FP64 form at most kFixItem
   int threads;           // CTA size of the gridding kernels
   size_t smem_tile;      // bytes of the staged tile
   int slab;              // planes of the padded tile in shared memory at a time (E[0]: all of them)

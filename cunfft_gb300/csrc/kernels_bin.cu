@@ -313,10 +313,10 @@ cudaError_t launch_binning(const Plan& p, const double* x, cudaStream_t st) {
                                                                            B.icount);
   // the scan of the interpolation's item counts: chunk 1, the counts themselves
   const bool sub_items = sub && tl.sub_items;
-  const ScanArgs nodes{B.count, tl.chunk, B.tile_off, B.item_off, B.num_items}, subs{B.icount, 1, B.iitem_off, B.iscratch, B.num_iitems};
+  const ScanArgs nodes{B.count, tl.item, B.tile_off, B.item_off, B.num_items}, subs{B.icount, 1, B.iitem_off, B.iscratch, B.num_iitems};
   k_scan_tiles<<<sub_items ? 2 : 1, 1024, 0, st>>>(nodes, subs, tl.tiles_total);
   if (B.M > 0) {
-    const ItemArgs ia{B.count, B.tile_off, B.item_off, tl.tiles_total, tl.chunk, B.items, B.scount, B.sub_pre, B.iitem_off, B.iitems,
+    const ItemArgs ia{B.count, B.tile_off, B.item_off, tl.tiles_total, tl.item, B.items, B.scount, B.sub_pre, B.iitem_off, B.iitems,
                       grid_for(tl.tiles_total, 256, p.num_sms), sub_items ? grid_for(nkeys, 256, p.num_sms) : 0};
     const int blocks = grid_for(B.M, 256, p.num_sms) + ia.tile_blocks + ia.sub_blocks;
     if (p.prec == kF64)

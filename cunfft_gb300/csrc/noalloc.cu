@@ -20,6 +20,7 @@
 // The array's device address is looked up once per device and cached; a device reset
 // (cudaDeviceReset) unloads the module, after which the cached address is stale, so
 // the entry point must not be used across a device reset.
+#include <algorithm>
 #include <mutex>
 #include <stdio.h>
 
@@ -30,8 +31,8 @@ namespace {
 
 constexpr int64_t kNaMaxNodes = int64_t(1) << 20;   // nodes per call
 constexpr int64_t kNaMaxTiles = int64_t(1) << 16;   // grid tiles per call
-constexpr int kNaChunk = 1024;                      // nodes per work item
-constexpr int64_t kNaMaxItems = kNaMaxTiles + kNaMaxNodes / kNaChunk + 1;
+constexpr int kNaChunk = 1024;                      // nodes per work item (FP64: kFixItem)
+constexpr int64_t kNaMaxItems = kNaMaxTiles + kNaMaxNodes / std::min(kNaChunk, kFixItem) + 1;
 
 // byte offsets of the scratch regions (each 256-byte aligned)
 constexpr size_t na_align(size_t v) { return (v + 255) / 256 * 256; }

@@ -164,8 +164,8 @@ static Tiling make_tiling(const Plan* p, const int* T, int chunk) {
   // CTAs better.  On the batched 2D workload 512 and 256 spread equally fast, 256 at 0.64
   // times the error against the FP64 form.
   const bool t2 = d == 2 && p->prec == kF32 && W <= 16;
-  // FP64 (fixed point): 512 nodes leave a cell's sum 53 bits below the largest sample
-  tl.chunk = chunk > 0 ? chunk : (p->prec == kF64 ? 512 : (d == 3 ? 1024 : (t2 ? 256 : 2048)));
+  tl.chunk = chunk > 0 ? chunk : (p->prec == kF64 ? kFixItem : (d == 3 ? 1024 : (t2 ? 256 : 2048)));
+  tl.item = p->prec == kF64 ? std::min(tl.chunk, kFixItem) : tl.chunk;
   tl.slab = tl.E[0];
   tl.ns = 1;  // no sub-bins unless the plan asks for them (plan_choose_tiling)
   return tl;
@@ -537,7 +537,7 @@ void plan_release(Plan* p) {
 static int ensure_bins(Plan* p, int64_t M) {
   Bins& B = p->bins;
   const int64_t tiles = p->tl.tiles_total;
-  const int64_t max_items = tiles + M / std::max(1, p->tl.chunk) + 1;
+  const int64_t max_items = tiles + M / std::max(1, p->tl.item) + 1;
   // sub-bin keys and their interpolation items (each sub-bin: at most count / kSubItem + 1)
   const int64_t keys = p->tl.sub_on ? tiles * p->tl.ns : 0;
   const int64_t max_iitems = keys > 0 && p->tl.sub_items ? keys + M / kSubItem + 1 : 0;
@@ -554,7 +554,7 @@ static int ensure_bins(Plan* p, int64_t M) {
     CG_TRY(check_cuda(p, plan_malloc(&B.count, sizeof(int32_t) * (capT + 1)), "cudaMalloc bins"));
     CG_TRY(check_cuda(p, plan_malloc(&B.tile_off, sizeof(int32_t) * (capT + 1)), "cudaMalloc bins"));
     CG_TRY(check_cuda(p, plan_malloc(&B.item_off, sizeof(int32_t) * (capT + 1)), "cudaMalloc bins"));
-    const int64_t cap_items = capT + capM / std::max(1, p->tl.chunk) + 1;
+    const int64_t cap_items = capT + capM / std::max(1, p->tl.item) + 1;
     CG_TRY(check_cuda(p, plan_malloc(&B.items, sizeof(int4) * cap_items), "cudaMalloc bins"));
     B.max_items = cap_items;
     if (keys > 0) {
@@ -592,6 +592,7 @@ static int item_nodes(const Plan* p) {
 
 static int rebin(Plan* p) {
   p->tl.chunk = item_nodes(p);
+  p->tl.item = p->prec == kF64 ? std::min(p->tl.chunk, kFixItem) : p->tl.chunk;
   CG_TRY(ensure_bins(p, p->M));
   p->bins.M = p->M;
   if (p->timing) cudaEventRecord(p->ev[6], p->stream);

@@ -190,7 +190,8 @@ int cunfft_x_set_stream(cunfft_x_plan *plan, void *stream);
 void *cunfft_x_get_stream(const cunfft_x_plan *plan);
 
 /** Tiling of the gridding kernels: tile extents T[d] (powers of two, each
- *  <= n_t) and the maximum number of nodes per work item.  Zeros keep the
+ *  <= n_t) and the maximum number of nodes per work item (FP64 plans take at most
+ *  512, which their sums' precision rests on).  Zeros keep the
  *  defaults.  Re-bins the current node set. */
 int cunfft_x_set_tiling(cunfft_x_plan *plan, const int *T, int chunk);
 
