@@ -135,6 +135,10 @@ __host__ __device__ constexpr int fix_plane_stride(int d, int W) {
 // leaves room for the sum of an item's samples, 2^9 of them at 53 bits below the largest.
 constexpr int kFixItem = 512;
 
+// 3D, FP64: up to this many taps the whole padded tile of 8 window starts fits in shared
+// memory; wider windows go through it in slabs of planes
+constexpr int kFixWholeW = 14;
+
 // Constants of the FP64 form's fixed-point gridding (kernels_fix.cuh), one set per plan.
 struct FixPar {
   uint64_t c60[kMaxDim];  // Gaussian: log2(e) / b_t in units of 2^-60 and of 2^-57

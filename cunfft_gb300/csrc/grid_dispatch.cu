@@ -5,7 +5,7 @@
 
 namespace cg {
 
-#define CG_DECL(W) cudaError_t grid_launch_w##W(const Plan&, bool, const void*, void*, cudaStream_t);
+#define CG_DECL(W) cudaError_t grid_launch_w##W(const Plan&, bool, bool, const void*, void*, cudaStream_t);
 CG_DECL(4) CG_DECL(6) CG_DECL(8) CG_DECL(10) CG_DECL(12) CG_DECL(14) CG_DECL(16) CG_DECL(18)
 CG_DECL(20) CG_DECL(22) CG_DECL(24) CG_DECL(26) CG_DECL(28) CG_DECL(30) CG_DECL(32)
 #undef CG_DECL
@@ -57,12 +57,12 @@ size_t gridding_smem_bytes(const Plan& p) {
   return p.tl.smem_tile + (a > b ? a : b);
 }
 
-static cudaError_t dispatch(const Plan& p, bool spread, const void* in, void* out, cudaStream_t st) {
+static cudaError_t dispatch(const Plan& p, bool spread, bool alone, const void* in, void* out, cudaStream_t st) {
   if (spread && p.tl.spread_kernel == CUNFFT_X_SPREAD_TENSOR) return grid_launch_spread_tc(p, in, out, st);
   if (!spread && p.tl.interp_kernel == CUNFFT_X_INTERP_TENSOR) return grid_launch_interp_tc(p, in, out, st);
   if (spread && p.tl.spread_kernel == CUNFFT_X_SPREAD_REGISTER) return grid_launch_spread_reg(p, in, out, st);
   switch (p.geo.W) {
-#define CG_CASE(W) case W: return grid_launch_w##W(p, spread, in, out, st);
+#define CG_CASE(W) case W: return grid_launch_w##W(p, spread, alone, in, out, st);
     CG_CASE(4) CG_CASE(6) CG_CASE(8) CG_CASE(10) CG_CASE(12) CG_CASE(14) CG_CASE(16) CG_CASE(18)
     CG_CASE(20) CG_CASE(22) CG_CASE(24) CG_CASE(26) CG_CASE(28) CG_CASE(30) CG_CASE(32)
 #undef CG_CASE
@@ -70,18 +70,18 @@ static cudaError_t dispatch(const Plan& p, bool spread, const void* in, void* ou
   }
 }
 
-cudaError_t launch_interp(const Plan& p, const void* g, void* f, cudaStream_t st) {
+cudaError_t launch_interp(const Plan& p, const void* g, void* f, bool alone, cudaStream_t st) {
   if (p.bins.M == 0) return cudaSuccess;
   cudaError_t e = cudaMemsetAsync(p.bins.work, 0, sizeof(int32_t), st);
   if (e != cudaSuccess) return e;
-  return dispatch(p, false, g, f, st);
+  return dispatch(p, false, alone, g, f, st);
 }
 
-cudaError_t launch_spread(const Plan& p, const void* f, void* g, cudaStream_t st) {
+cudaError_t launch_spread(const Plan& p, const void* f, void* g, bool alone, cudaStream_t st) {
   if (p.bins.M == 0) return cudaSuccess;
   cudaError_t e = cudaMemsetAsync(p.bins.work + 1, 0, sizeof(int32_t), st);
   if (e != cudaSuccess) return e;
-  return dispatch(p, true, f, g, st);
+  return dispatch(p, true, alone, f, g, st);
 }
 
 }  // namespace cg

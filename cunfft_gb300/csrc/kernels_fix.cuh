@@ -1,4 +1,9 @@
-// kernels_fix.cuh -- gridding of the FP64 form in 56-bit fixed point (fixmath.h).
+// kernels_fix.cuh -- gridding of the FP64 form's transforms in 56-bit fixed point (fixmath.h).
+//
+// The bits below a tile's largest value are the same for all of its cells, and taps have an
+// absolute error of 2^-54.  A transform's FFT mixes the cells anyway; the gridding stages alone,
+// whose callers may look at single small cells, stay in FP64 (k_interp and k_spread of
+// kernels_grid.cuh on the same tiles and items).
 //
 // Same method, work items and lane mapping as kernels_grid.cuh (the FP32 form's kernels);
 // the arithmetic is integer because GB300's FP64 pipe (about 2 multiply-adds per clock and
@@ -53,9 +58,6 @@ __host__ __device__ constexpr int fix_ctas(int d, int W, bool spread) {
 }
 // 1D spreading: node groups per warp (two windows of W <= 16 taps side by side)
 __host__ __device__ constexpr int fix_spread_groups(int W) { return W <= 16 ? 2 : 1; }
-// d = 3: up to this many taps the whole padded tile of 8 window starts fits in shared
-// memory; wider windows go through it in slabs of planes
-constexpr int kFixWholeW = 14;
 // d = 3 spreading in slabs: planes per slab, one for each pair of warps.  Full slabs and a
 // short last one: 33 planes (W = 26) as 8 + 8 + 8 + 8 + 1 instead of five of 7, where two of the
 // 16 warps idle.  With 40 nodes per batch: n = 128^3, M = 2^18 adjoint, W = 18 6.49 -> 6.06 ms,

@@ -1,5 +1,6 @@
 // kernels_grid.cuh -- tiled Gaussian gridding: interpolation (forward) and spreading (adjoint)
-// of the FP32 form (the FP64 form's kernels are in kernels_fix.cuh).
+// of the FP32 form, and of the FP64 form's stages on their own (its transforms grid in
+// kernels_fix.cuh).
 //
 // Method (the reference's, src/cunfft_kernel.cu:514-1149): node j touches the
 // (2m+2)^d grid points (u_t + l_t) mod n_t, l_t = 0..2m+1, with weight
@@ -41,13 +42,24 @@
 //    W = 18 1.45 -> 0.99 ms, W = 22 2.08 -> 1.46; W = 26 17.0 -> 2.24 and spreading 20.2 ->
 //    4.54 (one thread per node through global memory before).
 //  * Tap weights: one hardware exp2 per tap in the FP32 form; in the FP64 form the reference's
-//    fast-Gaussian-gridding recurrence (2 exp per node and dim, src/cunfft_kernel.cu:
-//    491-505), which keeps the scarce FP64 pipe on the taps.
+//    fast-Gaussian-gridding recurrence (src/cunfft_kernel.cu:491-505) from the middle tap
+//    outwards (4 exp per node and dim), which keeps the scarce FP64 pipe on the taps.
 #pragma once
 
 #include "runtime.h"
 
 namespace cg {
+
+// Compile-time extents and strides of the staged tile of elements C, and whether windows of W
+// taps go through it in slabs of planes.
+template <int D, int W, typename C>
+struct TileShape {
+  static constexpr bool F64 = sizeof(C) == 16;
+  static constexpr int S = F64 ? fix_row_stride(D, W) : fixed_row_stride(D, W);
+  static constexpr int PS = F64 ? fix_plane_stride(D, W) : fixed_plane_stride(D, W);
+  static constexpr int LAST = F64 ? fix_t_last(D) : fixed_t_last(D, W);
+  static constexpr bool SLAB = F64 ? D == 3 && W > kFixWholeW : grid_slabs(D, W);
+};
 
 // bits of the packed tile-local window start, per dimension
 __host__ __device__ constexpr int off_bits(int d) { return d == 1 ? 30 : (d == 2 ? 15 : 10); }
@@ -74,7 +86,9 @@ template <> struct WeightMath<float> {
 };
 
 template <> struct WeightMath<double> {
-  // FGG form: psi_l = phi * E^l * exp(-l^2/b), phi = exp(-c^2/b), E = exp(2c/b), c = m + fr.
+  // FGG form about the middle tap k = l - m = 0: psi_k = phi E^k exp(-k^2/b), phi = exp(-fr^2/b),
+  // E = exp(2 fr/b).  From the first tap on (c = m + fr in place of fr) every tap had the relative
+  // error of phi = exp(-c^2/b), some c^2/b = 20 roundings; here the large taps have a few.
   static __device__ __forceinline__ void taps(double fr, int m, const Geom& g, int t, int W, double* out) {
     if (g.window == kWinES) {  // exp(beta (sqrt(1 - y^2/alpha^2) - 1)), zero outside |y| < alpha
       const double beta = t == 0 ? g.es_beta[0] : (t == 1 ? g.es_beta[1] : g.es_beta[2]);
@@ -86,19 +100,19 @@ template <> struct WeightMath<double> {
       return;
     }
     const double b = t == 0 ? g.b[0] : (t == 1 ? g.b[1] : g.b[2]);
-    const double c = (double)m + fr;
     const double ib = 1.0 / b;
-    const double phi = exp(-(c * c) * ib);
-    const double E = exp(2.0 * c * ib);
-    const double q = exp(-ib);            // exp(-l^2/b) by the recurrence of src/cunfft.cu:60-76
-    double e = 1.0, gl = 1.0, qstep = q;  // gl = exp(-l^2/b), qstep = exp(-(2l+1)/b)
-    out[0] = phi;
+    const double E = exp(2.0 * fr * ib), Ei = exp(-2.0 * fr * ib);
+    const double q = exp(-ib);  // exp(-k^2/b) by the recurrence of src/cunfft.cu:60-76
+    double er = exp(-(fr * fr) * ib), el = er, gk = 1.0, qstep = q;  // phi E^k, phi E^-k, exp(-k^2/b), exp(-(2k+1)/b)
+    out[m] = er;
 #pragma unroll 4
-    for (int l = 1; l < W; ++l) {
-      e *= E;
-      gl *= qstep;
+    for (int k = 1; k <= m + 1; ++k) {
+      er *= E;
+      el *= Ei;
+      gk *= qstep;
       qstep *= q * q;
-      out[l] = phi * e * gl;
+      out[m + k] = er * gk;
+      if (k <= m) out[m - k] = el * gk;
     }
   }
 };
@@ -118,6 +132,11 @@ template <> struct WPair<float> {
   static __device__ __forceinline__ float2 make(float w) { return make_float2(w, w); }
 };
 __device__ __forceinline__ float2 cmul_addp(float2 acc, float2 ww, float2 v) { return __ffma2_rn(ww, v, acc); }
+template <> struct WPair<double> {
+  using t = double;
+  static __device__ __forceinline__ double make(double w) { return w; }
+};
+__device__ __forceinline__ double2 cmul_addp(double2 acc, double w, double2 v) { return cmul_add(acc, w, v); }
 
 // Asynchronous global -> shared copy of one complex element (cp.async, 8 or 16 bytes).
 template <typename C>
@@ -206,7 +225,7 @@ __device__ __forceinline__ int64_t row_gbase(const Geom& geo, const TileOrigin& 
 template <int D, int W, typename C>
 __device__ __forceinline__ void load_tile(C* tile, const C* __restrict__ gi, const Geom& geo, const Tiling& tl,
                                           const TileOrigin& o, int p_lo, int p_n) {
-  constexpr int S = fixed_row_stride(D, W), PS = fixed_plane_stride(D, W);
+  constexpr int S = TileShape<D, W, C>::S, PS = TileShape<D, W, C>::PS;
   const int E_last = tl.E[D - 1];
   const int64_t n_last = geo.n[D - 1], a_last = o.a[D - 1];
   if (D == 1) {
@@ -218,7 +237,7 @@ __device__ __forceinline__ void load_tile(C* tile, const C* __restrict__ gi, con
   // divisions: the staging was a third of the instructions of an item of some 80 nodes.
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int rows = D == 3 ? p_n * tl.E[1] : tile_rows<D>(tl), E1 = tl.E[1];
-  constexpr int NC = (fixed_t_last(D, W) + W - 1 + kWarp - 1) / kWarp;
+  constexpr int NC = (TileShape<D, W, C>::LAST + W - 1 + kWarp - 1) / kWarp;
   int64_t col[NC];
 #pragma unroll
   for (int c = 0; c < NC; ++c) col[c] = lane + c * kWarp < E_last ? wrap_up(a_last + lane + c * kWarp, n_last) : 0;
@@ -248,7 +267,7 @@ __device__ __forceinline__ void load_tile(C* tile, const C* __restrict__ gi, con
 template <int D, int W, typename C>
 __device__ __forceinline__ void flush_tile(const C* tile, C* __restrict__ gi, const Geom& geo, const Tiling& tl,
                                            const TileOrigin& o, int p_lo, int p_n) {
-  constexpr int S = fixed_row_stride(D, W), PS = fixed_plane_stride(D, W);
+  constexpr int S = TileShape<D, W, C>::S, PS = TileShape<D, W, C>::PS;
   const int E_last = tl.E[D - 1];
   const int64_t n_last = geo.n[D - 1], a_last = o.a[D - 1];
   const int rows = D == 3 ? p_n * tl.E[1] : tile_rows<D>(tl);
@@ -311,7 +330,7 @@ __host__ __device__ inline size_t grid_extra_smem(int d, int W, size_t real, int
 // Interpolation, d = 1..3
 // ---------------------------------------------------------------------------
 template <int D, int W, typename T>
-__global__ void __launch_bounds__(D == 3 && W > 16 ? 256 : 512) k_interp(const typename Cx<T>::t* __restrict__ g,
+__global__ void __launch_bounds__(sizeof(T) == 8 || (D == 3 && W > 16) ? 256 : 512) k_interp(const typename Cx<T>::t* __restrict__ g,
                                                 typename Cx<T>::t* __restrict__ f, Geom geo, Tiling tl, Bins bins) {
   using C = typename Cx<T>::t;
   constexpr int R = kWarp / W;           // rows (d >= 2) or nodes (d = 1) per warp pass
@@ -320,7 +339,7 @@ __global__ void __launch_bounds__(D == 3 && W > 16 ? 256 : 512) k_interp(const t
   constexpr int NB = nodes_per_warp_batch(D);
   constexpr int SH = off_bits(D);
   constexpr uint32_t MASK = (1u << SH) - 1u;
-  constexpr int S = fixed_row_stride(D, W), PS = fixed_plane_stride(D, W);
+  constexpr int S = TileShape<D, W, C>::S, PS = TileShape<D, W, C>::PS;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int4 cur;
   C* tile = reinterpret_cast<C*>(smem);
@@ -332,10 +351,10 @@ __global__ void __launch_bounds__(D == 3 && W > 16 ? 256 : 512) k_interp(const t
   const T* sfrac = reinterpret_cast<const T*>(bins.sfrac);
   const T norm = (T)geo.norm;
   const int qd = lane / D, td = lane - qd * D;  // (node, dim) of this lane in the weight pass
-  // d = 3, W > 16: lane i takes cells i, i + 32, ... of a plane's W x W window, so that no lane
-  // idles where W does not divide 32 (bank i mod 16, as S == W mod 16)
-  constexpr bool FLAT = D == 3 && R == 1;
-  constexpr bool SLAB = grid_slabs(D, W);
+  // d = 3, W > 16 (and slabs): lane i takes cells i, i + 32, ... of a plane's W x W window, so that
+  // no lane idles where W does not divide 32 (bank i mod 16, as S == W mod 16)
+  constexpr bool SLAB = TileShape<D, W, C>::SLAB;
+  constexpr bool FLAT = D == 3 && (R == 1 || SLAB);
   constexpr int NF = FLAT ? (W * W + kWarp - 1) / kWarp : 1;
   int fcell[NF];
 #pragma unroll
@@ -372,10 +391,14 @@ __global__ void __launch_bounds__(D == 3 && W > 16 ? 256 : 512) k_interp(const t
           nrec[lane] = pf_idx;
           nrec[NB + lane] = pf_off;
         }
-        for (int qt0 = 0; qt0 < nb * D; qt0 += R) {
-          const int qt = qt0 + r;
-          const float fr = __shfl_sync(0xffffffffu, pf_fr, min(qt, 31));
-          if (lane_on && qt < nb * D) wb[qt * W + l_last] = WeightMath<T>::tap(fr + (float)(geo.m - l_last), geo, qt % D);
+        if constexpr (sizeof(T) == 8) {
+          if (qd < nb) WeightMath<T>::taps(pf_fr, geo.m, geo, td, W, wb + (qd * D + td) * W);
+        } else {
+          for (int qt0 = 0; qt0 < nb * D; qt0 += R) {
+            const int qt = qt0 + r;
+            const float fr = __shfl_sync(0xffffffffu, pf_fr, min(qt, 31));
+            if (lane_on && qt < nb * D) wb[qt * W + l_last] = WeightMath<T>::tap(fr + (float)(geo.m - l_last), geo, qt % D);
+          }
         }
         // fetch the next batch's records while this batch runs
         const int bn = bs + nwarps * nbw;
@@ -510,7 +533,7 @@ __global__ void __launch_bounds__(D == 3 && W > 16 ? 256 : 512) k_interp(const t
 // Spreading, d = 1..3
 // ---------------------------------------------------------------------------
 template <int D, int W, typename T>
-__global__ void __launch_bounds__(512) k_spread(const typename Cx<T>::t* __restrict__ f,
+__global__ void __launch_bounds__(sizeof(T) == 8 ? 256 : 512) k_spread(const typename Cx<T>::t* __restrict__ f,
                                                 typename Cx<T>::t* __restrict__ g, Geom geo, Tiling tl, Bins bins) {
   using C = typename Cx<T>::t;
   constexpr int R = kWarp / W;
@@ -519,12 +542,12 @@ __global__ void __launch_bounds__(512) k_spread(const typename Cx<T>::t* __restr
   constexpr int NBC = kNodesPerCtaBatch;
   constexpr int SH = off_bits(D);
   constexpr uint32_t MASK = (1u << SH) - 1u;
-  constexpr int S = fixed_row_stride(D, W), PS = fixed_plane_stride(D, W);
+  constexpr int S = TileShape<D, W, C>::S, PS = TileShape<D, W, C>::PS;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int4 cur;
   C* tile = reinterpret_cast<C*>(smem);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  constexpr bool SLAB = grid_slabs(D, W);
+  constexpr bool SLAB = TileShape<D, W, C>::SLAB;
   const int tile_elems = D == 1 ? tl.E[0] : (D == 2 ? tl.E[0] * S : tl.slab * PS);
   // d = 1: one private tile copy per warp (copy 0 is `tile`)
   const size_t extra = D == 1 ? (size_t)(nwarps - 1) * tl.smem_tile : 0;

@@ -151,7 +151,7 @@ extern "C" int cunfft_x_spread_noalloc(int d, const int64_t* N, const int64_t* n
   B.valid = 1;
   p.M = M;
   p.x = x;
-  if ((e = launch_binning(p, x, st)) != cudaSuccess || (e = launch_spread(p, f, g, st)) != cudaSuccess) {
+  if ((e = launch_binning(p, x, st)) != cudaSuccess || (e = launch_spread(p, f, g, true, st)) != cudaSuccess) {
     fprintf(stderr, "cunfft_x_spread_noalloc: launch failed: %s\n", cudaGetErrorString(e));
     return CUNFFT_X_CUDA_ERROR;
   }

@@ -682,7 +682,7 @@ int plan_forward(Plan* p, const void* fhat, void* f) {
   rec(p, 0);
   CG_TRY(forward_grid(p, fhat, p->fft_fwd_ext ? p->fft_fwd_ext : p->fft));
   rec(p, 2);
-  CG_TRY(check_cuda(p, launch_interp(*p, p->g, f, p->stream), "interpolation kernel"));
+  CG_TRY(check_cuda(p, launch_interp(*p, p->g, f, false, p->stream), "interpolation kernel"));
   rec(p, 3);
   return set_status(p, CUNFFT_X_SUCCESS, nullptr);
 }
@@ -694,7 +694,7 @@ int plan_adjoint(Plan* p, const void* f, void* fhat) {
   rec(p, 0);
   CG_TRY(check_cuda(p, cudaMemsetAsync(p->g, 0, elem_bytes(p) * p->geo.ntot * p->geo.batch, p->stream),
                     "clear grid"));
-  CG_TRY(check_cuda(p, launch_spread(*p, f, p->g, p->stream), "spreading kernel"));
+  CG_TRY(check_cuda(p, launch_spread(*p, f, p->g, false, p->stream), "spreading kernel"));
   rec(p, 1);
   if (p->fx_on)
     CG_TRY(check_cuda(p, launch_fft_fix(*p, nullptr, p->g, true, p->stream), "adjoint FFT"));
@@ -749,14 +749,14 @@ int plan_interp_only(Plan* p, const void* g, void* f) {
   if (!p->nodes_set) return set_status(p, CUNFFT_X_NODES_NOT_SET, "interp: nodes not set");
   if (!p->bins.valid) CG_TRY(rebin(p));
   CG_TRY(prepare_interp(p));
-  CG_TRY(check_cuda(p, launch_interp(*p, g, f, p->stream), "interpolation kernel"));
+  CG_TRY(check_cuda(p, launch_interp(*p, g, f, true, p->stream), "interpolation kernel"));
   return set_status(p, CUNFFT_X_SUCCESS, nullptr);
 }
 
 int plan_spread_only(Plan* p, const void* f, void* g) {
   if (!p->nodes_set) return set_status(p, CUNFFT_X_NODES_NOT_SET, "spread: nodes not set");
   if (!p->bins.valid) CG_TRY(rebin(p));
-  CG_TRY(check_cuda(p, launch_spread(*p, f, g, p->stream), "spreading kernel"));
+  CG_TRY(check_cuda(p, launch_spread(*p, f, g, true, p->stream), "spreading kernel"));
   return set_status(p, CUNFFT_X_SUCCESS, nullptr);
 }
 
@@ -826,7 +826,7 @@ int plan_autotune(Plan* p, int reps) {
       return -1.f;
     }
     auto run = [&]() {
-      return spread ? launch_spread(*p, scratch_f, p->g, p->stream) : launch_interp(*p, p->g, scratch_f, p->stream);
+      return spread ? launch_spread(*p, scratch_f, p->g, false, p->stream) : launch_interp(*p, p->g, scratch_f, false, p->stream);
     };
     if (run() != cudaSuccess) return -1.f;
     cudaEventRecord(a, p->stream);

@@ -168,8 +168,9 @@ cudaError_t launch_fft_fix(const Plan& p, const void* fhat, void* g, bool inv, c
 void fft_fix_prepare(Plan& p);
 void fft_fix_release(Plan& p);
 cudaError_t launch_roc_adjoint(const Plan& p, const void* g, void* fhat, cudaStream_t st);
-cudaError_t launch_interp(const Plan& p, const void* g, void* f, cudaStream_t st);
-cudaError_t launch_spread(const Plan& p, const void* f, void* g, cudaStream_t st);
+// alone: not followed or preceded by the plan's FFT (the FP64 form then grids in FP64)
+cudaError_t launch_interp(const Plan& p, const void* g, void* f, bool alone, cudaStream_t st);
+cudaError_t launch_spread(const Plan& p, const void* f, void* g, bool alone, cudaStream_t st);
 cudaError_t launch_interp_grad(const Plan& p, const void* g, const void* grad_f, double* grad_x, cudaStream_t st);
 cudaError_t launch_ndft_forward(const Plan& p, const double* x, const void* fhat, void* f, cudaStream_t st);
 cudaError_t launch_ndft_adjoint(const Plan& p, const double* x, const void* f, void* fhat, cudaStream_t st,

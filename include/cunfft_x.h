@@ -143,7 +143,9 @@ int cunfft_x_cg(cunfft_x_plan* plan, int stage, int64_t it, int64_t iters, doubl
  *  (batch*n_total complex, plan precision): interpolation g -> f and
  *  spreading f -> g (spreading accumulates into g; clear it first).  g needs only
  *  the alignment of its element type (8 bytes for FP32 complex); 16-byte aligned
- *  grids take the wider accesses. */
+ *  grids take the wider accesses.  FP64 plans: in FP64 arithmetic, every value with
+ *  its own relative precision (the transforms grid in fixed point relative to a
+ *  tile's largest value, which their FFT mixes anyway). */
 int cunfft_x_interp(cunfft_x_plan *plan, const void *g, void *f);
 int cunfft_x_spread(cunfft_x_plan *plan, const void *f, void *g);
 
