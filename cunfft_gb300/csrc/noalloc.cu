@@ -109,6 +109,16 @@ extern "C" int cunfft_x_spread_noalloc(int d, const int64_t* N, const int64_t* n
     fprintf(stderr, "cunfft_x_spread_noalloc: %s\n", p.last_msg);
     return s;
   }
+  // 2D FP64 plans take tiles of 16 rows for their CTAs per SM; here 32 halve the tiles of the
+  // grids that would need too many
+  if (d == 2 && precision == kF64 && p.tl.tiles_total > kNaMaxTiles) {
+    const int T32[3] = {32, 0, 0};
+    s = plan_choose_tiling(&p, T32, kNaChunk);
+    if (s != CUNFFT_X_SUCCESS) {
+      fprintf(stderr, "cunfft_x_spread_noalloc: %s\n", p.last_msg);
+      return s;
+    }
+  }
   p.tl.sub_on = 0;  // spreading needs the nodes in tile order only: no sub-bins, no room for them
   p.tl.sub_items = 0;
   p.tl.ns = 1;

@@ -170,12 +170,11 @@ int cunfft_x_spread(cunfft_x_plan *plan, const void *f, void *g);
  *  Its scratch (node bins, tile counts, work queue) is one fixed device array
  *  inside the library, about 58 MB, which every GPU that loads the library holds
  *  until the process exits.  Limits: M <= 1048576 nodes and at most 65536 grid
- *  tiles, the tiles being prod_t ceil(n_t / T_t) for the plan's default tile
- *  extents T.  With m <= 7, 3D tiles are 8 x 8 x 16 (FP32) or 4 x 8 x 16 (FP64), so
- *  n = 256^3 needs 16384 or 32768 tiles and fits, n = 512^3 does not; wider windows
- *  (m >= 8) use 8 x 4 x 8 (FP32) or 4 x 4 x 8 (FP64) tiles in 3D, and a tile whose
- *  padded copy would not fit shared memory is halved along dimension 0.  2D tiles
- *  are 64 x 64 grid points (FP32, m <= 7) or 32 x 64, 1D tiles 2048.
+ *  tiles, the tiles being prod_t ceil(n_t / T_t) for tile extents T.  3D tiles are
+ *  8 x 8 x 16 grid points (FP64, and FP32 with m <= 7), so n = 256^3 needs 16384 tiles
+ *  and fits, n = 512^3 does not; FP32 with m >= 8 uses 8 x 4 x 8 tiles, of fewer planes
+ *  where the padded copy would not fit shared memory (m <= 11).  2D tiles are 64 x 64
+ *  (FP32, m <= 7) or 32 x 64, 1D tiles at most 2048 (FP32) or 1024 (FP64) grid points.
  *  Larger requests return CUNFFT_X_INVALID_ARGUMENT with a message on stderr and
  *  do no device work.  M = 0 leaves g unchanged.
  *
