@@ -92,6 +92,7 @@ static void free_bins(Plan* p) {
   B.count = nullptr; B.tile_off = nullptr; B.item_off = nullptr; B.items = nullptr;
   B.scount = nullptr; B.sub_pre = nullptr; B.icount = nullptr; B.iitem_off = nullptr; B.iscratch = nullptr;
   B.iitems = nullptr;
+  B.max_items = 0;
   B.max_iitems = 0;
   p->bins_capacity_M = -1;
   p->bins_capacity_tiles = -1;
@@ -534,48 +535,6 @@ void plan_release(Plan* p) {
   p->M_inst = nullptr;
 }
 
-static int ensure_bins(Plan* p, int64_t M) {
-  Bins& B = p->bins;
-  const int64_t tiles = p->tl.tiles_total;
-  const int64_t max_items = tiles + M / std::max(1, p->tl.item) + 1;
-  // sub-bin keys and their interpolation items (each sub-bin: at most count / kSubItem + 1)
-  const int64_t keys = p->tl.sub_on ? tiles * p->tl.ns : 0;
-  const int64_t max_iitems = keys > 0 && p->tl.sub_items ? keys + M / kSubItem + 1 : 0;
-  const size_t real = elem_bytes(p) / 2;
-  if (M > p->bins_capacity_M || tiles > p->bins_capacity_tiles || max_items > B.max_items ||
-      keys > p->bins_capacity_keys || max_iitems > B.max_iitems || p->bins_capacity_M < 0) {
-    const int64_t capM = std::max<int64_t>(M, 1), capT = tiles;
-    free_bins(p);
-    CG_TRY(check_cuda(p, plan_malloc(&B.sidx, sizeof(int32_t) * capM), "cudaMalloc bins"));
-    CG_TRY(check_cuda(p, plan_malloc(&B.soff, sizeof(int32_t) * capM), "cudaMalloc bins"));
-    CG_TRY(check_cuda(p, plan_malloc(&B.sfrac, real * p->geo.d * capM), "cudaMalloc bins"));
-    CG_TRY(check_cuda(p, plan_malloc(&B.tile_rank, sizeof(int2) * capM), "cudaMalloc bins"));
-    CG_TRY(check_cuda(p, plan_malloc(&B.fperm, elem_bytes(p) * capM), "cudaMalloc bins"));
-    CG_TRY(check_cuda(p, plan_malloc(&B.count, sizeof(int32_t) * (capT + 1)), "cudaMalloc bins"));
-    CG_TRY(check_cuda(p, plan_malloc(&B.tile_off, sizeof(int32_t) * (capT + 1)), "cudaMalloc bins"));
-    CG_TRY(check_cuda(p, plan_malloc(&B.item_off, sizeof(int32_t) * (capT + 1)), "cudaMalloc bins"));
-    const int64_t cap_items = capT + capM / std::max(1, p->tl.item) + 1;
-    CG_TRY(check_cuda(p, plan_malloc(&B.items, sizeof(int4) * cap_items), "cudaMalloc bins"));
-    B.max_items = cap_items;
-    if (keys > 0) {
-      CG_TRY(check_cuda(p, plan_malloc(&B.scount, sizeof(int32_t) * (keys + 1)), "cudaMalloc bins"));
-      CG_TRY(check_cuda(p, plan_malloc(&B.sub_pre, sizeof(int32_t) * keys), "cudaMalloc bins"));
-    }
-    if (max_iitems > 0) {
-      const int64_t cap_ii = keys + capM / kSubItem + 1;
-      CG_TRY(check_cuda(p, plan_malloc(&B.icount, sizeof(int32_t) * (capT + 1)), "cudaMalloc bins"));
-      CG_TRY(check_cuda(p, plan_malloc(&B.iitem_off, sizeof(int32_t) * (capT + 1)), "cudaMalloc bins"));
-      CG_TRY(check_cuda(p, plan_malloc(&B.iscratch, sizeof(int32_t) * (capT + 1)), "cudaMalloc bins"));
-      CG_TRY(check_cuda(p, plan_malloc(&B.iitems, sizeof(int4) * cap_ii), "cudaMalloc bins"));
-      B.max_iitems = cap_ii;
-    }
-    p->bins_capacity_M = capM;
-    p->bins_capacity_tiles = capT;
-    p->bins_capacity_keys = keys;
-  }
-  return CUNFFT_X_SUCCESS;
-}
-
 // Nodes per work item for M nodes: the default, less where that would leave SMs without an
 // item (a few thousand nodes, or a grid of few tiles), down to one batch of the gridding
 // kernels.  Four items per SM even out their lengths; every item stages or adds out its
@@ -588,6 +547,58 @@ static int item_nodes(const Plan* p) {
   int c = 32;
   while (c < most && c * (int64_t)p->num_sms * 4 < p->M) c *= 2;
   return c;
+}
+
+// Most items beyond one per tile that any node set of at most M nodes has: shorter items for
+// fewer nodes (item_nodes) make at most four per SM.
+static int64_t most_items(const Plan* p, int64_t M) {
+  if (p->chunk_override > 0) return M / std::max(1, p->tl.item);
+  return std::max(M / make_tiling(p, p->tl.T, 0).item, (int64_t)p->num_sms * 4);
+}
+
+// Room for M nodes on the current tiling.  Capacities only grow, and hold every smaller node
+// set as well, so that alternating node sets allocate once.
+static int ensure_bins(Plan* p, int64_t M) {
+  Bins& B = p->bins;
+  const int64_t tiles = p->tl.tiles_total;
+  const int64_t max_items = tiles + most_items(p, M) + 1;
+  // sub-bin keys and their interpolation items (each sub-bin: at most count / kSubItem + 1)
+  const int64_t keys = p->tl.sub_on ? tiles * p->tl.ns : 0;
+  const int64_t max_iitems = keys > 0 && p->tl.sub_items ? keys + M / kSubItem + 1 : 0;
+  const size_t real = elem_bytes(p) / 2;
+  if (M > p->bins_capacity_M || tiles > p->bins_capacity_tiles || max_items > B.max_items ||
+      keys > p->bins_capacity_keys || max_iitems > B.max_iitems || p->bins_capacity_M < 0) {
+    const int64_t capM = std::max({M, p->bins_capacity_M, (int64_t)1}), capT = std::max(tiles, p->bins_capacity_tiles);
+    const int64_t cap_items = std::max(capT + most_items(p, capM) + 1, B.max_items);
+    const int64_t cap_keys = std::max(keys, p->bins_capacity_keys), cap_iitems = B.max_iitems;
+    free_bins(p);
+    CG_TRY(check_cuda(p, plan_malloc(&B.sidx, sizeof(int32_t) * capM), "cudaMalloc bins"));
+    CG_TRY(check_cuda(p, plan_malloc(&B.soff, sizeof(int32_t) * capM), "cudaMalloc bins"));
+    CG_TRY(check_cuda(p, plan_malloc(&B.sfrac, real * p->geo.d * capM), "cudaMalloc bins"));
+    CG_TRY(check_cuda(p, plan_malloc(&B.tile_rank, sizeof(int2) * capM), "cudaMalloc bins"));
+    CG_TRY(check_cuda(p, plan_malloc(&B.fperm, elem_bytes(p) * capM), "cudaMalloc bins"));
+    CG_TRY(check_cuda(p, plan_malloc(&B.count, sizeof(int32_t) * (capT + 1)), "cudaMalloc bins"));
+    CG_TRY(check_cuda(p, plan_malloc(&B.tile_off, sizeof(int32_t) * (capT + 1)), "cudaMalloc bins"));
+    CG_TRY(check_cuda(p, plan_malloc(&B.item_off, sizeof(int32_t) * (capT + 1)), "cudaMalloc bins"));
+    CG_TRY(check_cuda(p, plan_malloc(&B.items, sizeof(int4) * cap_items), "cudaMalloc bins"));
+    B.max_items = cap_items;
+    if (cap_keys > 0) {
+      CG_TRY(check_cuda(p, plan_malloc(&B.scount, sizeof(int32_t) * (cap_keys + 1)), "cudaMalloc bins"));
+      CG_TRY(check_cuda(p, plan_malloc(&B.sub_pre, sizeof(int32_t) * cap_keys), "cudaMalloc bins"));
+    }
+    if (max_iitems > 0 || cap_iitems > 0) {
+      const int64_t cap_ii = std::max(cap_keys + capM / kSubItem + 1, cap_iitems);
+      CG_TRY(check_cuda(p, plan_malloc(&B.icount, sizeof(int32_t) * (capT + 1)), "cudaMalloc bins"));
+      CG_TRY(check_cuda(p, plan_malloc(&B.iitem_off, sizeof(int32_t) * (capT + 1)), "cudaMalloc bins"));
+      CG_TRY(check_cuda(p, plan_malloc(&B.iscratch, sizeof(int32_t) * (capT + 1)), "cudaMalloc bins"));
+      CG_TRY(check_cuda(p, plan_malloc(&B.iitems, sizeof(int4) * cap_ii), "cudaMalloc bins"));
+      B.max_iitems = cap_ii;
+    }
+    p->bins_capacity_M = capM;
+    p->bins_capacity_tiles = capT;
+    p->bins_capacity_keys = cap_keys;
+  }
+  return CUNFFT_X_SUCCESS;
 }
 
 static int rebin(Plan* p) {
