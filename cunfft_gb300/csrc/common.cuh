@@ -155,10 +155,10 @@ struct Tiling {
   int E[kMaxDim];        // padded extent per dim = T_t + W - 1
   int S;                 // shared-memory row stride (elements) for the innermost dim
   int R1;                // rows per plane (E[d-2] for d = 3, unused otherwise)
+  int item;              // max nodes per work item: chunk, in the FP64 form at most kFixItem
   int64_t tiles_per_inst;
   int64_t tiles_total;   // batch * tiles_per_inst
   int chunk;             // max nodes per work item, as asked for
-  int item;              // max nodes per work item: chunk, in the FP64 form at most kFixItem
   int threads;           // CTA size of the gridding kernels
   size_t smem_tile;      // bytes of the staged tile
   int slab;              // planes of the padded tile in shared memory at a time (E[0]: all of them)
