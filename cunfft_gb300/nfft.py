@@ -10,6 +10,7 @@ Layouts (as the reference): nodes ``x`` float64 (M, d) in [-0.5, 0.5);
 coefficients (batch, *N) row-major with frequency k_t at index k_t + N_t//2;
 samples (M,).
 """
+import collections
 import ctypes
 
 import torch
@@ -22,12 +23,23 @@ def _ptr(t):
 
 
 class NFFT:
+    # plans with a private stream per device: with one alone nothing has to be held (making another
+    # waits for the work of those before it)
+    _private_plans = collections.Counter()
+    # tensors held before an event is spent on them (one is a gap of some 15 us in the stream)
+    _HELD_BYTES = 256 << 20
+
     def __init__(self, N, n=None, m=6, precision="f64", batch=1, device=None, stream=None, window="gaussian"):
         self._host_refs = []  # host tensors in flight in host-buffer transforms
-        # The device tensors of the last forward and adjoint transform.  A plan on the default
-        # stream runs on a private one, which torch's allocator does not know: a block that the
-        # caller drops while the plan still writes it could go to another plan's next output.
+        # Device tensors that calls in flight use.  A plan on the default stream runs on a private
+        # one, which torch's allocator does not know: a block that the caller drops while the plan
+        # still uses it could go to the next output of another such plan (_keep; not of the same
+        # plan, and torch's default stream waits for private ones.  The allocator cannot be told
+        # of the stream, which tensors may outlive.)
         self._live = {}
+        self._open, self._open_calls = [], 1
+        self._pending = collections.deque()
+        self._private = None
         self._lib = nat.lib()
         self.N = [int(v) for v in N]
         self.d = len(self.N)
@@ -45,10 +57,17 @@ class NFFT:
             Na = (ctypes.c_int64 * self.d)(*self.N)
             na = (ctypes.c_int64 * self.d)(*(n if n is not None else [0] * self.d))
             h = ctypes.c_void_p()
+            private = stream.cuda_stream == 0
+            self._index = torch.cuda.current_device()
+            NFFT._private_plans[self._index] += private
             st = self._lib.cunfft_x_plan_create(ctypes.byref(h), self.d, Na, na, self.m, self.precision,
                                                 self.batch, ctypes.c_void_p(stream.cuda_stream))
+            if st != nat.SUCCESS:
+                NFFT._private_plans[self._index] -= private
             nat.check(st)
         self._h = h
+        if private:
+            self._private = torch.cuda.ExternalStream(self._lib.cunfft_x_get_stream(h), device=self.device)
         self.n = self._grid_sizes(n)
         self.N_total = 1
         for v in self.N:
@@ -86,9 +105,13 @@ class NFFT:
             raise ValueError("M_inst must have one count per instance summing to x.shape[0]")
         arr = (ctypes.c_int64 * self.batch)(*M_inst)
         nat.check(self._lib.cunfft_x_set_nodes(self._h, _ptr(x), arr), self._h)
+        if self.x is not None and self.x.data_ptr() != x.data_ptr():
+            self._keep(self.x)
         self.x = x  # keep the storage alive: the plan reads it
         self.M_inst = M_inst
         self.M = M
+        call = 2 * (self.cdtype.itemsize * (self.batch * self.N_total + M) + 8 * self.d * M)
+        self._open_calls = max(1, NFFT._HELD_BYTES // max(1, call))
         return self
 
     # ------------------------------------------------------------ transforms
@@ -104,9 +127,37 @@ class NFFT:
             raise ValueError("f has the wrong size")
         return f
 
-    def _keep(self, what, a, out):
-        # without the autograd graph of an input
-        self._live[what] = (a.detach() if a.grad_fn is not None else a, out.detach() if out.grad_fn is not None else out)
+    def _keep(self, *tensors):
+        """Hold tensors while the work issued so far may use them: in batches of about _HELD_BYTES,
+        until a later batch finds the work before it done, synchronize() or close()."""
+        if self._private is None or NFFT._private_plans[self._index] < 2:
+            return
+        self._open.append([t.detach() if t.requires_grad else t for t in tensors])  # without an autograd graph
+        if len(self._open) < self._open_calls:
+            return
+        done = torch.cuda.Event()
+        done.record(self._private)
+        self._pending.append((done, self._open))
+        self._open = []
+        if not torch.cuda.is_current_stream_capturing():  # no query while a graph is captured
+            while self._pending and self._pending[0][0].query():
+                self._pending.popleft()
+
+    def _keep_last(self, what, a, out):
+        """Hold a transform's tensors at least until the next one of its kind."""
+        if self._private is None or NFFT._private_plans[self._index] < 2:
+            return
+        if a.requires_grad or out.requires_grad:
+            a, out = a.detach(), out.detach()
+        before = self._live.get(what)
+        self._live[what] = (a, out)
+        if before is not None and (before[0] is not a or before[1] is not out):  # a loop's fixed buffers stay
+            self._keep(*before)
+
+    def _release(self):
+        self._pending.clear()
+        self._live.clear()
+        self._open = []
 
     def _coef_shape(self):
         return ([self.batch] if self.batch > 1 else []) + self.N
@@ -115,14 +166,14 @@ class NFFT:
         fhat = self._coef(fhat)
         f = out if out is not None else torch.empty(self.M, dtype=self.cdtype, device=self.device)
         nat.check(self._lib.cunfft_x_forward(self._h, _ptr(fhat), _ptr(f)), self._h)
-        self._keep("forward", fhat, f)
+        self._keep_last("forward", fhat, f)
         return f
 
     def adjoint(self, f, out=None):
         f = self._samples(f)
         fh = out if out is not None else torch.empty(self._coef_shape(), dtype=self.cdtype, device=self.device)
         nat.check(self._lib.cunfft_x_adjoint(self._h, _ptr(f), _ptr(fh)), self._h)
-        self._keep("adjoint", f, fh)
+        self._keep_last("adjoint", f, fh)
         return fh
 
     # ------------------------------------------------ host buffers, overlapped copies
@@ -148,11 +199,14 @@ class NFFT:
             if len(M_inst) != self.batch or sum(M_inst) != M:
                 raise ValueError("M_inst must have one count per instance summing to the node count")
             arr = (ctypes.c_int64 * self.batch)(*M_inst)
-            self.M_inst, self.M, self.x = M_inst, M, None
+            bound, self.x = self.x, None
+            self.M_inst, self.M = M_inst, M
         self._host(fhat, self.cdtype, self.batch * self.N_total, "fhat")
         self._host(out, self.cdtype, self.M, "out")
         nat.check(self._lib.cunfft_x_forward_host(self._h, _ptr(x), arr, _ptr(fhat), _ptr(out)), self._h)
         self._host_refs.extend([x, fhat, out])
+        if x is not None and bound is not None:
+            self._keep(bound)
         return out
 
     def adjoint_host(self, f, out):
@@ -167,24 +221,28 @@ class NFFT:
         """forward() replayed from a captured CUDA graph (fixed buffers fhat, out)."""
         fhat = self._coef(fhat)
         nat.check(self._lib.cunfft_x_forward_graph(self._h, _ptr(fhat), _ptr(out)), self._h)
+        self._keep_last("forward graph", fhat, out)
         return out
 
     def adjoint_graph(self, f, out):
         """adjoint() replayed from a captured CUDA graph (fixed buffers f, out)."""
         f = self._samples(f)
         nat.check(self._lib.cunfft_x_adjoint_graph(self._h, _ptr(f), _ptr(out)), self._h)
+        self._keep_last("adjoint graph", f, out)
         return out
 
     def ndft_forward(self, fhat):
         fhat = fhat.to(torch.complex128).contiguous()
         f = torch.empty(self.M, dtype=torch.complex128, device=self.device)
         nat.check(self._lib.cunfft_x_ndft_forward(self._h, _ptr(fhat), _ptr(f)), self._h)
+        self._keep(fhat, f)
         return f
 
     def ndft_adjoint(self, f):
         f = f.to(torch.complex128).contiguous()
         fh = torch.empty(self._coef_shape(), dtype=torch.complex128, device=self.device)
         nat.check(self._lib.cunfft_x_ndft_adjoint(self._h, _ptr(f), _ptr(fh)), self._h)
+        self._keep(f, fh)
         return fh
 
     def ndft_adjoint_at(self, f, kidx):
@@ -194,6 +252,7 @@ class NFFT:
         out = torch.empty(self.batch * kidx.numel(), dtype=torch.complex128, device=self.device)
         nat.check(self._lib.cunfft_x_ndft_adjoint_at(self._h, _ptr(f), _ptr(kidx), kidx.numel(), _ptr(out)),
                   self._h)
+        self._keep(f, kidx, out)
         return out
 
     def node_gradient(self, fhat, grad_f):
@@ -201,12 +260,14 @@ class NFFT:
         grad_f = self._samples(grad_f)
         gx = torch.empty(self.M, self.d, dtype=torch.float64, device=self.device)
         nat.check(self._lib.cunfft_x_node_gradient(self._h, _ptr(fhat), _ptr(grad_f), _ptr(gx)), self._h)
+        self._keep(fhat, grad_f, gx)
         return gx
 
     def interp(self, g, out=None):
         g = g.to(self.cdtype).contiguous()
         f = out if out is not None else torch.empty(self.M, dtype=self.cdtype, device=self.device)
         nat.check(self._lib.cunfft_x_interp(self._h, _ptr(g), _ptr(f)), self._h)
+        self._keep(g, f)
         return f
 
     def spread(self, f, g=None):
@@ -214,6 +275,7 @@ class NFFT:
         if g is None:
             g = torch.zeros(([self.batch] if self.batch > 1 else []) + self.n, dtype=self.cdtype, device=self.device)
         nat.check(self._lib.cunfft_x_spread(self._h, _ptr(f), _ptr(g)), self._h)
+        self._keep(f, g)
         return g
 
     # ---------------------------------------------------------------- tuning
@@ -282,7 +344,7 @@ class NFFT:
     def synchronize(self):
         nat.check(self._lib.cunfft_x_synchronize(self._h), self._h)
         self._host_refs = []  # host buffers of finished host-buffer transforms
-        self._live.clear()
+        self._release()
 
     def grid(self):
         """The plan's oversampled grid as a tensor view (batch, *n)."""
@@ -297,7 +359,9 @@ class NFFT:
         if getattr(self, "_h", None):
             self._lib.cunfft_x_plan_destroy(self._h)
             self._h = None
-            self._live.clear()
+            if self._private is not None:
+                NFFT._private_plans[self._index] -= 1
+            self._release()
 
     def __del__(self):
         try:
