@@ -17,9 +17,17 @@
 // rows (forward: 8 rows of a thread) or computed once per CTA (adjoint: a product over the
 // nodes of 32 rows by 32 pairs, 4 rows by 1 pair per thread); they come from sincospi of the
 // exactly reduced argument, followed by at most 31 (forward) or 15 (adjoint) rotations.
-// Measured at N = 64^2, M = 4096: forward 98 us (one rotation and one product per term, on
-// 16 CTAs, before: 2.28 ms), adjoint 90 us (one sincospi per term before: 9.70 ms); two
+// Measured at N = 64^2, M = 4096: forward 82 us (one rotation and one product per term, on
+// 16 CTAs, before: 2.28 ms), adjoint 69 us (one sincospi per term before: 9.70 ms); two
 // operations per term alone take 56 us at the measured rate.
+//
+// Sums that are split over CTAs go through a buffer of partial sums (at most some 10 MB, kept
+// by the plan) and are added in a fixed order, so that results repeat bit by bit: 153 us for
+// both directions at N = 64^2, M = 4096, 140 with atomic additions.  A result that is not finite
+// is summed again term by term: the sums and differences of pairs turn infinities into NaN, and
+// overflow before the terms do.
+#include <algorithm>
+
 #include "runtime.h"
 
 namespace cg {
@@ -103,10 +111,94 @@ __device__ __forceinline__ double ndft_turn(const NdftGroup<D>& q, const double*
   return t;
 }
 
+__device__ __forceinline__ bool finite2(double2 v) { return isfinite(v.x) && isfinite(v.y); }
+
+// f_j term by term
 template <int D>
+__device__ __noinline__ double2 ndft_node(const Geom& geo, const double2* __restrict__ fh, const double* __restrict__ x) {
+  double2 acc = make_double2(0.0, 0.0);
+  for (int64_t i = 0; i < geo.Ntot; ++i) {
+    double t = 0.0;
+    int64_t rem = i;
+#pragma unroll
+    for (int s = D - 1; s >= 0; --s) {
+      t += turn((double)(rem % geo.N[s] - geo.N[s] / 2), x[s]);
+      rem /= geo.N[s];
+    }
+    acc = cfma(fh[i], cis2pi(-t), acc);
+  }
+  return acc;
+}
+
+// coefficient i of an instance term by term
+template <int D>
+__device__ __noinline__ double2 ndft_coef(const Geom& geo, const double* __restrict__ x, const double2* __restrict__ f,
+                                          int64_t j0, int64_t j1, int64_t i) {
+  double k[D];
+#pragma unroll
+  for (int s = D - 1; s >= 0; --s) {
+    k[s] = (double)(i % geo.N[s] - geo.N[s] / 2);
+    i /= geo.N[s];
+  }
+  double2 acc = make_double2(0.0, 0.0);
+  for (int64_t j = j0; j < j1; ++j) {
+    double t = 0.0;
+#pragma unroll
+    for (int s = 0; s < D; ++s) t += turn(k[s], x[j * D + s]);
+    acc = cfma(f[j], cis2pi(t), acc);
+  }
+  return acc;
+}
+
+// Partial sums [splits][n] added in a fixed order (warp w of the CTA adds every eighth split of 32
+// results, then the warps' sums); what is not finite again term by term.
+template <int D, bool ADJ>
+__global__ void __launch_bounds__(256) k_ndft_add(const double* __restrict__ x, const double2* __restrict__ in,
+                                                  const double2* __restrict__ part, double2* __restrict__ out, Geom geo,
+                                                  const int32_t* __restrict__ inst_off, int64_t n, int splits) {
+  __shared__ double2 sum[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int64_t e0 = blockIdx.x * (int64_t)32; e0 < n; e0 += (int64_t)gridDim.x * 32) {
+    const int64_t e = e0 + lane;
+    double2 v = make_double2(0.0, 0.0);
+    if (e < n) {
+#pragma unroll 8
+      for (int s = warp; s < splits; s += 8) {
+        const double2 p = part[s * n + e];
+        v.x += p.x;
+        v.y += p.y;
+      }
+    }
+    sum[warp][lane] = v;
+    __syncthreads();
+    if (warp == 0 && e < n) {
+#pragma unroll
+      for (int w = 1; w < 8; ++w) {
+        v.x += sum[w][lane].x;
+        v.y += sum[w][lane].y;
+      }
+      if (!finite2(v)) {
+        if (ADJ) {
+          const int64_t inst = e / geo.Ntot;
+          v = ndft_coef<D>(geo, x, in, inst_off[inst], inst_off[inst + 1], e - inst * geo.Ntot);
+        } else {
+          int inst = 0;
+          while (inst + 1 < geo.batch && inst_off[inst + 1] <= e) ++inst;
+          v = ndft_node<D>(geo, in + inst * geo.Ntot, x + e * D);
+        }
+      }
+      out[e] = v;
+    }
+    __syncthreads();
+  }
+}
+
+// SPLIT: partial sums of split blockIdx.z to part [split][total], total nodes of all instances
+template <int D, bool SPLIT>
 __global__ void __launch_bounds__(128) k_ndft_forward(const double* __restrict__ x, const double2* __restrict__ fhat,
                                                       double2* __restrict__ f, Geom geo,
-                                                      const int32_t* __restrict__ inst_off, NdftRows nr) {
+                                                      const int32_t* __restrict__ inst_off, NdftRows nr,
+                                                      double2* __restrict__ part, int64_t total) {
   constexpr int R = kNdftRowsF;
   __shared__ double2 sd[kNdftPairs][R][2];  // a+ + a-, -i (a+ - a-)
   const int inst = blockIdx.y;
@@ -114,7 +206,7 @@ __global__ void __launch_bounds__(128) k_ndft_forward(const double* __restrict__
   const double2* fh = fhat + (int64_t)inst * geo.Ntot;
   const int64_t NL = geo.N[D - 1];
   const int half = (int)(nr.B / 2);
-  // row groups g0 .. g1 - 1 of this split (partial sums added atomically)
+  // row groups g0 .. g1 - 1 of this split
   const int64_t ng = nr.slow * nr.groups, span = (ng + gridDim.z - 1) / gridDim.z;
   const int64_t g0 = (int64_t)blockIdx.z * span, g1 = min(ng, g0 + span);
   for (int64_t jb = j0 + (int64_t)blockIdx.x * blockDim.x; jb < j1; jb += (int64_t)gridDim.x * blockDim.x) {
@@ -164,20 +256,17 @@ __global__ void __launch_bounds__(128) k_ndft_forward(const double* __restrict__
       }
     }
     if (on) {
-      if (gridDim.z == 1) {
-        f[j] = acc;
-      } else {
-        atomicAdd(&f[j].x, acc.x);
-        atomicAdd(&f[j].y, acc.y);
-      }
+      if (SPLIT) part[blockIdx.z * total + j] = acc;
+      else f[j] = finite2(acc) ? acc : ndft_node<D>(geo, fh, x + j * D);
     }
   }
 }
 
-template <int D>
+template <int D, bool SPLIT>
 __global__ void __launch_bounds__(256) k_ndft_adjoint(const double* __restrict__ x, const double2* __restrict__ f,
                                                       double2* __restrict__ fhat, Geom geo,
-                                                      const int32_t* __restrict__ inst_off, NdftRows nr) {
+                                                      const int32_t* __restrict__ inst_off, NdftRows nr,
+                                                      double2* __restrict__ part) {
   constexpr int NJ = kNdftNodesA, RB = kNdftRowsA, SEG = 16;
   __shared__ double2 scs[NJ][kNdftPairs];  // cos, sin of a node's pairs
   __shared__ double2 sc[NJ][RB];           // f_j times the row's phase
@@ -186,7 +275,7 @@ __global__ void __launch_bounds__(256) k_ndft_adjoint(const double* __restrict__
   const int64_t NL = geo.N[D - 1];
   const int half = (int)(nr.B / 2);
   const NdftGroup<D> q = ndft_group<D>(geo, nr, blockIdx.x);
-  // nodes of this split (partial sums added atomically)
+  // nodes of this split
   const int64_t span = (j1 - j0 + gridDim.z - 1) / gridDim.z;
   const int64_t n_lo = j0 + (int64_t)blockIdx.z * span, n_hi = min(j1, n_lo + span);
   double2 A[4], Bv[4];
@@ -237,7 +326,7 @@ __global__ void __launch_bounds__(256) k_ndft_adjoint(const double* __restrict__
       }
     }
   }
-  double2* out = fhat + (int64_t)inst * geo.Ntot;
+  double2* out = (SPLIT ? part + blockIdx.z * (geo.Ntot * geo.batch) : fhat) + (int64_t)inst * geo.Ntot;
   for (int r = 0; r < 4; ++r) {
     const int rr = warp * 4 + r;
     if (rr >= q.n || lane >= half) continue;
@@ -246,12 +335,7 @@ __global__ void __launch_bounds__(256) k_ndft_adjoint(const double* __restrict__
     const double2 vp = make_double2(A[r].x - Bv[r].y, A[r].y + Bv[r].x), vm = make_double2(A[r].x + Bv[r].y, A[r].y - Bv[r].x);
     auto put = [&](int64_t c, double2 v) {
       if (c >= NL) return;
-      if (gridDim.z == 1) {
-        out[row + c] = v;
-      } else {
-        atomicAdd(&out[row + c].x, v.x);
-        atomicAdd(&out[row + c].y, v.y);
-      }
+      out[row + c] = SPLIT || finite2(v) ? v : ndft_coef<D>(geo, x, f, j0, j1, row + c);
     };
     put(cp, vp);
     put(cm, vm);
@@ -312,7 +396,7 @@ __global__ void __launch_bounds__(256) k_ndft_adjoint_at(const double* __restric
 }
 
 // Few selected coefficients would occupy a few SMs only: split the inner sum over up to 4 CTAs per SM, at least 4096 terms each.
-static int ndft_splits(const Plan& p, int64_t blocks, int64_t inner) {
+static int ndft_at_splits(const Plan& p, int64_t blocks, int64_t inner) {
   const int64_t want = (int64_t)p.num_sms * 4;
   if (blocks >= want) return 1;
   int64_t s = (want + blocks - 1) / blocks;
@@ -343,36 +427,102 @@ static int64_t max_nodes(const Plan& p) {
   return m;
 }
 
-cudaError_t launch_ndft_forward(const Plan& p, const double* x, const void* fhat, void* f, cudaStream_t st) {
-  const int64_t maxM = max_nodes(p);
-  if (maxM == 0) return cudaSuccess;
-  const NdftRows nr = ndft_rows(p.geo, kNdftRowsF);
-  const int64_t ng = nr.slow * nr.groups, want = (int64_t)p.num_sms * 6;
+// Launch of one direction: CTAs along nodes (forward) or row groups (adjoint), splits, results.
+struct NdftLaunch {
+  NdftRows nr;
+  int threads;
+  int64_t bx, splits, results;
+};
+
+static NdftLaunch ndft_launch_forward(const Plan& p) {
+  NdftLaunch l;
+  const int64_t maxM = max_nodes(p), want = (int64_t)p.num_sms * 6;
+  l.nr = ndft_rows(p.geo, kNdftRowsF);
+  const int64_t ng = l.nr.slow * l.nr.groups;
   // one warp per CTA until there are enough CTAs to spread evenly over the SMs
-  const int threads = (maxM + 127) / 128 * p.geo.batch * ng >= want ? 128 : 32;
-  int64_t bx = (maxM + threads - 1) / threads;
-  if (bx > (int64_t)p.num_sms * 16) bx = (int64_t)p.num_sms * 16;
-  int64_t splits = (want + bx * p.geo.batch - 1) / (bx * p.geo.batch);
-  if (splits > ng) splits = ng;
-  if (splits > 65535) splits = 65535;
-  if (splits > 1) {
-    const cudaError_t e = cudaMemsetAsync(f, 0, sizeof(double2) * p.M, st);
-    if (e != cudaSuccess) return e;
+  l.threads = (maxM + 127) / 128 * p.geo.batch * ng >= want ? 128 : 32;
+  l.bx = std::max<int64_t>(1, (maxM + l.threads - 1) / l.threads);
+  if (l.bx > (int64_t)p.num_sms * 16) l.bx = (int64_t)p.num_sms * 16;
+  l.splits = (want + l.bx * p.geo.batch - 1) / (l.bx * p.geo.batch);
+  if (l.splits > ng) l.splits = ng;
+  if (l.splits > 65535) l.splits = 65535;
+  l.results = p.M;
+  return l;
+}
+
+static NdftLaunch ndft_launch_adjoint(const Plan& p) {
+  NdftLaunch l;
+  const int64_t maxM = max_nodes(p);
+  l.nr = ndft_rows(p.geo, kNdftRowsA);
+  l.threads = 256;
+  l.bx = l.nr.slow * l.nr.groups;
+  // nodes split so that two CTAs run per SM, at least four nodes each
+  l.splits = (int64_t)p.num_sms * 2 / (l.bx * p.geo.batch);
+  if (l.splits > (maxM + 3) / 4) l.splits = (maxM + 3) / 4;
+  if (l.splits < 1) l.splits = 1;
+  l.results = p.geo.Ntot * p.geo.batch;
+  return l;
+}
+
+// Splits of a direction's sums: as planned where the plan has room for the partial sums (made for
+// both directions at once), 1 where it cannot be had, and while the stream is captured (the graph
+// may outlive the room).
+static int64_t ndft_splits(Plan& p, const NdftLaunch& l, cudaStream_t st) {
+  if (l.splits <= 1) return 1;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return 1;
   }
-  const dim3 grid((unsigned)bx, (unsigned)p.geo.batch, (unsigned)splits);
-  auto kern = p.geo.d == 1 ? k_ndft_forward<1> : (p.geo.d == 2 ? k_ndft_forward<2> : k_ndft_forward<3>);
-  kern<<<grid, threads, 0, st>>>(x, (const double2*)fhat, (double2*)f, p.geo, p.bins.inst_off, nr);
+  if (l.splits * l.results <= p.nd_cap) return l.splits;
+  const NdftLaunch f = ndft_launch_forward(p), a = ndft_launch_adjoint(p);
+  const int64_t need = std::max(f.splits > 1 ? f.splits * f.results : 0, a.splits > 1 ? a.splits * a.results : 0);
+  ndft_release(p);
+  if (plan_malloc(&p.nd_part, sizeof(double2) * (size_t)need) != cudaSuccess) {
+    cudaGetLastError();
+    p.nd_part = nullptr;
+    return 1;
+  }
+  p.nd_cap = need;
+  return l.splits;
+}
+
+void ndft_release(Plan& p) {
+  cudaFree(p.nd_part);
+  p.nd_part = nullptr;
+  p.nd_cap = 0;
+}
+
+template <bool ADJ>
+static cudaError_t add_partial_sums(const Plan& p, const double* x, const void* in, void* out, int64_t n, int splits,
+                                    cudaStream_t st) {
+  int64_t blocks = (n + 31) / 32;
+  if (blocks > (int64_t)p.num_sms * 8) blocks = (int64_t)p.num_sms * 8;
+  auto kern = p.geo.d == 1 ? k_ndft_add<1, ADJ> : (p.geo.d == 2 ? k_ndft_add<2, ADJ> : k_ndft_add<3, ADJ>);
+  kern<<<(unsigned)blocks, 256, 0, st>>>(x, (const double2*)in, (const double2*)p.nd_part, (double2*)out, p.geo, p.bins.inst_off,
+                                         n, splits);
   return cudaGetLastError();
 }
 
-cudaError_t launch_ndft_adjoint(const Plan& p, const double* x, const void* f, void* fhat, cudaStream_t st,
+cudaError_t launch_ndft_forward(Plan& p, const double* x, const void* fhat, void* f, cudaStream_t st) {
+  if (max_nodes(p) == 0) return cudaSuccess;
+  const NdftLaunch l = ndft_launch_forward(p);
+  const int64_t splits = ndft_splits(p, l, st);
+  const dim3 grid((unsigned)l.bx, (unsigned)p.geo.batch, (unsigned)splits);
+  auto kern = splits > 1 ? (p.geo.d == 1 ? k_ndft_forward<1, true> : (p.geo.d == 2 ? k_ndft_forward<2, true> : k_ndft_forward<3, true>))
+                         : (p.geo.d == 1 ? k_ndft_forward<1, false> : (p.geo.d == 2 ? k_ndft_forward<2, false> : k_ndft_forward<3, false>));
+  kern<<<grid, l.threads, 0, st>>>(x, (const double2*)fhat, (double2*)f, p.geo, p.bins.inst_off, l.nr, (double2*)p.nd_part, p.M);
+  if (splits > 1) return add_partial_sums<false>(p, x, fhat, f, l.results, (int)splits, st);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_ndft_adjoint(Plan& p, const double* x, const void* f, void* fhat, cudaStream_t st,
                                 const int64_t* kidx, int64_t nsel) {
-  const int64_t maxM = max_nodes(p);
   if (kidx) {
     if (nsel == 0) return cudaSuccess;
     int64_t bx = (nsel + 255) / 256;
     if (bx > (int64_t)p.num_sms * 8) bx = (int64_t)p.num_sms * 8;
-    const int splits = ndft_splits(p, bx * p.geo.batch, maxM);
+    const int splits = ndft_at_splits(p, bx * p.geo.batch, max_nodes(p));
     if (splits > 1) {
       const cudaError_t e = cudaMemsetAsync(fhat, 0, sizeof(double2) * nsel * p.geo.batch, st);
       if (e != cudaSuccess) return e;
@@ -381,19 +531,13 @@ cudaError_t launch_ndft_adjoint(const Plan& p, const double* x, const void* f, v
     k_ndft_adjoint_at<<<grid, 256, 0, st>>>(x, (const double2*)f, (double2*)fhat, p.geo, p.bins.inst_off, kidx, nsel);
     return cudaGetLastError();
   }
-  const NdftRows nr = ndft_rows(p.geo, kNdftRowsA);
-  const int64_t ng = nr.slow * nr.groups;
-  // nodes split so that two CTAs run per SM, at least four nodes each
-  int64_t splits = (int64_t)p.num_sms * 2 / (ng * p.geo.batch);
-  if (splits > (maxM + 3) / 4) splits = (maxM + 3) / 4;
-  if (splits < 1) splits = 1;
-  if (splits > 1) {
-    const cudaError_t e = cudaMemsetAsync(fhat, 0, sizeof(double2) * p.geo.Ntot * p.geo.batch, st);
-    if (e != cudaSuccess) return e;
-  }
-  const dim3 grid((unsigned)ng, (unsigned)p.geo.batch, (unsigned)splits);
-  auto kern = p.geo.d == 1 ? k_ndft_adjoint<1> : (p.geo.d == 2 ? k_ndft_adjoint<2> : k_ndft_adjoint<3>);
-  kern<<<grid, 256, 0, st>>>(x, (const double2*)f, (double2*)fhat, p.geo, p.bins.inst_off, nr);
+  const NdftLaunch l = ndft_launch_adjoint(p);
+  const int64_t splits = ndft_splits(p, l, st);
+  const dim3 grid((unsigned)l.bx, (unsigned)p.geo.batch, (unsigned)splits);
+  auto kern = splits > 1 ? (p.geo.d == 1 ? k_ndft_adjoint<1, true> : (p.geo.d == 2 ? k_ndft_adjoint<2, true> : k_ndft_adjoint<3, true>))
+                         : (p.geo.d == 1 ? k_ndft_adjoint<1, false> : (p.geo.d == 2 ? k_ndft_adjoint<2, false> : k_ndft_adjoint<3, false>));
+  kern<<<grid, l.threads, 0, st>>>(x, (const double2*)f, (double2*)fhat, p.geo, p.bins.inst_off, l.nr, (double2*)p.nd_part);
+  if (splits > 1) return add_partial_sums<true>(p, x, f, fhat, l.results, (int)splits, st);
   return cudaGetLastError();
 }
 

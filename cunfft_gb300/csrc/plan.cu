@@ -525,6 +525,7 @@ void plan_release(Plan* p) {
   cudaFree(p->roc_tab);
   p->roc_tab = nullptr;
   fft_fix_release(*p);
+  ndft_release(*p);
   if (p->own_fft && p->fft) cufftDestroy(p->fft);
   p->fft = 0;
   for (int i = 0; i < 8; ++i)

@@ -70,6 +70,8 @@ struct Plan {
   void* g_out[2] = {nullptr, nullptr};
   uint64_t g_gen[2] = {0, 0};
   uint64_t node_gen = 0;  // bumped by every node binding / tiling change
+  void* nd_part = nullptr;  // partial sums of the direct NDFT (complex128), created by the first split sum
+  int64_t nd_cap = 0;
   HostPath* hp = nullptr; // created by the first host-buffer transform
   // tensor-core interpolation: the grid's padded FP16 hi/lo planes, their per-plane
   // inverse scales and their TMA map, created before its first launch (interp_tc_prepare)
@@ -172,8 +174,9 @@ cudaError_t launch_roc_adjoint(const Plan& p, const void* g, void* fhat, cudaStr
 cudaError_t launch_interp(const Plan& p, const void* g, void* f, bool alone, cudaStream_t st);
 cudaError_t launch_spread(const Plan& p, const void* f, void* g, bool alone, cudaStream_t st);
 cudaError_t launch_interp_grad(const Plan& p, const void* g, const void* grad_f, double* grad_x, cudaStream_t st);
-cudaError_t launch_ndft_forward(const Plan& p, const double* x, const void* fhat, void* f, cudaStream_t st);
-cudaError_t launch_ndft_adjoint(const Plan& p, const double* x, const void* f, void* fhat, cudaStream_t st,
+cudaError_t launch_ndft_forward(Plan& p, const double* x, const void* fhat, void* f, cudaStream_t st);
+void ndft_release(Plan& p);
+cudaError_t launch_ndft_adjoint(Plan& p, const double* x, const void* f, void* fhat, cudaStream_t st,
                                 const int64_t* kidx = nullptr, int64_t nsel = 0);
 cudaError_t launch_cg(const Plan& p, int stage, int64_t it, int64_t iters, double lam, double tol, const void* b, void* x,
                       void* r, void* pv, void* ap, double* scal, int32_t* stop, cudaStream_t st);

@@ -105,7 +105,10 @@ int cunfft_x_forward_graph(cunfft_x_plan *plan, const void *f_hat, void *f);
 int cunfft_x_adjoint_graph(cunfft_x_plan *plan, const void *f, void *f_hat);
 
 /** Direct NDFT and adjoint NDFT on the bound nodes, always in FP64 with
- *  complex128 buffers, whatever the plan precision (the error yardstick). */
+ *  complex128 buffers, whatever the plan precision (the error yardstick).  The same
+ *  call gives the same bits.  Sums of few outputs are split over CTAs through a buffer
+ *  of at most some 10 MB that the plan makes at the first such call and keeps (none
+ *  while the stream is captured: one CTA per output block then). */
 int cunfft_x_ndft_forward(cunfft_x_plan *plan, const void *f_hat, void *f);
 int cunfft_x_ndft_adjoint(cunfft_x_plan *plan, const void *f, void *f_hat);
 
