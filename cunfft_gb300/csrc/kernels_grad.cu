@@ -23,8 +23,7 @@ __global__ void __launch_bounds__(128) k_interp_grad(const double* __restrict__ 
                                                      const typename Cx<T>::t* __restrict__ grad_f,
                                                      double* __restrict__ grad_x, Geom geo,
                                                      const int32_t* __restrict__ inst_off, int64_t M) {
-  using C = typename Cx<T>::t;
-  const int d = geo.d, W = geo.W;
+  const int d = geo.d;
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < M; j += (int64_t)gridDim.x * blockDim.x) {
     int inst = 0;
     if (geo.batch > 1) {
@@ -35,69 +34,7 @@ __global__ void __launch_bounds__(128) k_interp_grad(const double* __restrict__ 
       }
       inst = lo;
     }
-    const C* gi = g + (int64_t)inst * geo.ntot;
-    T w[kMaxDim][kMaxTaps], dw[kMaxDim][kMaxTaps];
-    int64_t u[kMaxDim] = {0, 0, 0};
-    for (int t = 0; t < d; ++t) {
-      const double xt = x[j * d + t];
-      const double nx = __dmul_rn(xt, (double)geo.n[t]);
-      u[t] = (int64_t)__double2ll_rn(nx) - (signbit(xt) ? 1 : 0) - geo.m;
-      const double c = __dsub_rn(nx, (double)u[t]);
-      if (geo.window == kWinES) {
-        // phi = exp(beta (s - 1)), s = sqrt(1 - y^2/alpha^2); dphi/dy = -phi beta y / (alpha^2 s)
-        const double beta = geo.es_beta[t];
-        for (int l = 0; l < W; ++l) {
-          const double y = c - (double)l, z = 1.0 - (y * y) * geo.es_ia2;
-          const double s = z > 0.0 ? sqrt(z) : 0.0;
-          const double e = z > 0.0 ? exp(beta * (s - 1.0)) : 0.0;
-          w[t][l] = (T)e;
-          dw[t][l] = z > 0.0 ? (T)(-e * beta * y * geo.es_ia2 / s * (double)geo.n[t]) : (T)0;
-        }
-      } else {
-        const double ib = 1.0 / geo.b[t];
-        for (int l = 0; l < W; ++l) {
-          const double y = c - (double)l;
-          const double e = exp(-(y * y) * ib);
-          w[t][l] = (T)e;
-          dw[t][l] = (T)(-2.0 * y * ib * e * (double)geo.n[t]);
-        }
-      }
-    }
-    for (int t = d; t < kMaxDim; ++t) {
-      w[t][0] = (T)1;
-      dw[t][0] = (T)0;
-    }
-    const int W1 = d >= 2 ? W : 1, W2 = d >= 3 ? W : 1;
-    // partial sums: p[t] = sum g * (derivative in dim t, plain weights elsewhere)
-    T pr[kMaxDim] = {0, 0, 0}, pi[kMaxDim] = {0, 0, 0};
-    for (int l0 = 0; l0 < W; ++l0) {
-      const int64_t i0 = wrap_n(u[0] + l0, geo.n[0]);
-      for (int l1 = 0; l1 < W1; ++l1) {
-        const int64_t i1 = d >= 2 ? wrap_n(u[1] + l1, geo.n[1]) : 0;
-        // inner sums over the last dimension: plain and derivative weights
-        T ar = 0, ai = 0, br = 0, bi = 0;
-        for (int l2 = 0; l2 < W2; ++l2) {
-          const int64_t i2 = d >= 3 ? wrap_n(u[2] + l2, geo.n[2]) : 0;
-          int64_t gidx = i0;
-          if (d >= 2) gidx = gidx * geo.n[1] + i1;
-          if (d >= 3) gidx = gidx * geo.n[2] + i2;
-          const C v = gi[gidx];
-          const T a = d >= 3 ? w[2][l2] : (T)1, b = d >= 3 ? dw[2][l2] : (T)0;
-          ar += a * v.x; ai += a * v.y;
-          br += b * v.x; bi += b * v.y;
-        }
-        // (ar, ai): plain in last dim; (br, bi): derivative in dim 2
-        const T w1 = d >= 2 ? w[1][l1] : (T)1, dw1 = d >= 2 ? dw[1][l1] : (T)0;
-        const T w0 = w[0][l0], dw0 = dw[0][l0];
-        pr[0] += dw0 * w1 * ar; pi[0] += dw0 * w1 * ai;
-        if (d >= 2) { pr[1] += w0 * dw1 * ar; pi[1] += w0 * dw1 * ai; }
-        if (d >= 3) { pr[2] += w0 * w1 * br; pi[2] += w0 * w1 * bi; }
-      }
-    }
-    const C gf = grad_f[j];
-    const double nrm = geo.norm;
-    for (int t = 0; t < d; ++t)
-      grad_x[j * d + t] = nrm * ((double)gf.x * (double)pr[t] + (double)gf.y * (double)pi[t]);
+    grad_node_global<T>(x + j * d, g + (int64_t)inst * geo.ntot, grad_f[j], grad_x + j * d, geo);
   }
 }
 

@@ -20,8 +20,75 @@ constexpr int kGradThreads = 128;
 // mantissa and a power of two.
 struct GradPar {
   uint64_t mant[kMaxDim];  // |c| = mant 2^-63 2^e, mant in [2^62, 2^63)
-  float scale[kMaxDim];    // 2^e / 2^56, negative
+  float scale[kMaxDim];    // 2^e / 2^60, negative
 };
+
+// Gradient of one node (coordinates x) on its instance's grid, through global memory.
+template <typename T>
+__device__ __noinline__ void grad_node_global(const double* __restrict__ x, const typename Cx<T>::t* __restrict__ gi,
+                                              typename Cx<T>::t gf, double* __restrict__ out, const Geom& geo) {
+  using C = typename Cx<T>::t;
+  const int d = geo.d, W = geo.W;
+  T w[kMaxDim][kMaxTaps], dw[kMaxDim][kMaxTaps];
+  int64_t u[kMaxDim] = {0, 0, 0};
+  for (int t = 0; t < d; ++t) {
+    const double xt = x[t];
+    const double nx = __dmul_rn(xt, (double)geo.n[t]);
+    u[t] = (int64_t)__double2ll_rn(nx) - (signbit(xt) ? 1 : 0) - geo.m;
+    const double c = __dsub_rn(nx, (double)u[t]);
+    if (geo.window == kWinES) {
+      // phi = exp(beta (s - 1)), s = sqrt(1 - y^2/alpha^2); dphi/dy = -phi beta y / (alpha^2 s)
+      const double beta = geo.es_beta[t];
+      for (int l = 0; l < W; ++l) {
+        const double y = c - (double)l, z = 1.0 - (y * y) * geo.es_ia2;
+        const double s = z > 0.0 ? sqrt(z) : 0.0;
+        const double e = z > 0.0 ? exp(beta * (s - 1.0)) : 0.0;
+        w[t][l] = (T)e;
+        dw[t][l] = z > 0.0 ? (T)(-e * beta * y * geo.es_ia2 / s * (double)geo.n[t]) : (T)0;
+      }
+    } else {
+      const double ib = 1.0 / geo.b[t];
+      for (int l = 0; l < W; ++l) {
+        const double y = c - (double)l;
+        const double e = exp(-(y * y) * ib);
+        w[t][l] = (T)e;
+        dw[t][l] = (T)(-2.0 * y * ib * e * (double)geo.n[t]);
+      }
+    }
+  }
+  for (int t = d; t < kMaxDim; ++t) {
+    w[t][0] = (T)1;
+    dw[t][0] = (T)0;
+  }
+  const int W1 = d >= 2 ? W : 1, W2 = d >= 3 ? W : 1;
+  // partial sums: p[t] = sum g * (derivative in dim t, plain weights elsewhere)
+  T pr[kMaxDim] = {0, 0, 0}, pi[kMaxDim] = {0, 0, 0};
+  for (int l0 = 0; l0 < W; ++l0) {
+    const int64_t i0 = wrap_n(u[0] + l0, geo.n[0]);
+    for (int l1 = 0; l1 < W1; ++l1) {
+      const int64_t i1 = d >= 2 ? wrap_n(u[1] + l1, geo.n[1]) : 0;
+      // inner sums over the last dimension: plain and derivative weights
+      T ar = 0, ai = 0, br = 0, bi = 0;
+      for (int l2 = 0; l2 < W2; ++l2) {
+        const int64_t i2 = d >= 3 ? wrap_n(u[2] + l2, geo.n[2]) : 0;
+        int64_t gidx = i0;
+        if (d >= 2) gidx = gidx * geo.n[1] + i1;
+        if (d >= 3) gidx = gidx * geo.n[2] + i2;
+        const C v = gi[gidx];
+        const T a = d >= 3 ? w[2][l2] : (T)1, b = d >= 3 ? dw[2][l2] : (T)0;
+        ar += a * v.x; ai += a * v.y;
+        br += b * v.x; bi += b * v.y;
+      }
+      // (ar, ai): plain in last dim; (br, bi): derivative in dim 2
+      const T w1 = d >= 2 ? w[1][l1] : (T)1, dw1 = d >= 2 ? dw[1][l1] : (T)0;
+      const T w0 = w[0][l0], dw0 = dw[0][l0];
+      pr[0] += dw0 * w1 * ar; pi[0] += dw0 * w1 * ai;
+      if (d >= 2) { pr[1] += w0 * dw1 * ar; pi[1] += w0 * dw1 * ai; }
+      if (d >= 3) { pr[2] += w0 * w1 * br; pi[2] += w0 * w1 * bi; }
+    }
+  }
+  for (int t = 0; t < d; ++t) out[t] = geo.norm * ((double)gf.x * (double)pr[t] + (double)gf.y * (double)pi[t]);
+}
 
 template <int D, int W>
 __global__ void __launch_bounds__(kGradThreads)
@@ -45,12 +112,19 @@ __global__ void __launch_bounds__(kGradThreads)
       const int j = bins.sidx[k];
       const uint32_t off = (uint32_t)bins.soff[k];
       float w[D][W], dw[D][W];
+      bool moved = false;
 #pragma unroll
       for (int t = 0; t < D; ++t) {
         const double xt = x[(int64_t)j * D + t], n = (double)geo.n[t];
         const double nx = __dmul_rn(xt, n);
-        const double fr = __dsub_rn(nx, (double)(__double2ll_rn(nx) - (signbit(xt) ? 1 : 0)));
-        if (!(fabs(fr) < 2.0)) {  // the coordinate is not finite
+        const int64_t u = __double2ll_rn(nx) - (signbit(xt) ? 1 : 0);
+        const double fr = __dsub_rn(nx, (double)u);
+        const bool finite = fabs(fr) < 2.0;
+        int64_t s = u - geo.m;  // window start, as the binning found it unless x has changed since
+        if (s < 0) s += geo.n[t];
+        if (s < 0 || s >= geo.n[t]) s = wrap_n(s, geo.n[t]);
+        moved |= finite && s != o.a[t] + ((off >> (SH * t)) & MASK);
+        if (!finite) {
           for (int l = 0; l < W; ++l) w[t][l] = dw[t][l] = __int_as_float(0x7fc00000);
         } else if (geo.window == kWinES) {
           for (int l = 0; l < W; ++l) {
@@ -73,6 +147,10 @@ __global__ void __launch_bounds__(kGradThreads)
             dw[t][l] = y < 0 ? -d : d;
           }
         }
+      }
+      if (moved) {  // another window than the tile's: the coordinates count, as in the other form
+        grad_node_global<float>(x + (int64_t)j * D, g + o.inst * geo.ntot, grad_f[j], grad_x + (int64_t)j * D, geo);
+        continue;
       }
       float pr[D], pi[D], wl[W], dl[W];
 #pragma unroll
