@@ -25,7 +25,7 @@ struct GradPar {
 
 // Gradient of one node (coordinates x) on its instance's grid, through global memory.
 template <typename T>
-__device__ __noinline__ void grad_node_global(const double* __restrict__ x, const typename Cx<T>::t* __restrict__ gi,
+__device__ __forceinline__ void grad_node_global(const double* __restrict__ x, const typename Cx<T>::t* __restrict__ gi,
                                               typename Cx<T>::t gf, double* __restrict__ out, const Geom& geo) {
   using C = typename Cx<T>::t;
   const int d = geo.d, W = geo.W;
@@ -90,6 +90,12 @@ __device__ __noinline__ void grad_node_global(const double* __restrict__ x, cons
   for (int t = 0; t < d; ++t) out[t] = geo.norm * ((double)gf.x * (double)pr[t] + (double)gf.y * (double)pi[t]);
 }
 
+// ... out of line, for the few nodes of a tile that need it
+static __device__ __noinline__ void grad_node_moved(const double* __restrict__ x, const float2* __restrict__ gi, float2 gf,
+                                                    double* __restrict__ out, const Geom& geo) {
+  grad_node_global<float>(x, gi, gf, out, geo);
+}
+
 template <int D, int W>
 __global__ void __launch_bounds__(kGradThreads)
     k_grad_tile(const double* __restrict__ x, const float2* __restrict__ g, const float2* __restrict__ grad_f,
@@ -149,7 +155,7 @@ __global__ void __launch_bounds__(kGradThreads)
         }
       }
       if (moved) {  // another window than the tile's: the coordinates count, as in the other form
-        grad_node_global<float>(x + (int64_t)j * D, g + o.inst * geo.ntot, grad_f[j], grad_x + (int64_t)j * D, geo);
+        grad_node_moved(x + (int64_t)j * D, g + o.inst * geo.ntot, grad_f[j], grad_x + (int64_t)j * D, geo);
         continue;
       }
       float pr[D], pi[D], wl[W], dl[W];
