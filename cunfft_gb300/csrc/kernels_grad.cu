@@ -10,7 +10,7 @@
 // No reference counterpart (the reference has no differentiable transform).
 // FP64 node reduction and weights; accumulation in the plan's real type.  The FP32 form runs
 // on staged tiles (kernels_grad_tile.cuh); the kernel here, one thread per node with the
-// grid read through L1/L2, takes the FP64 form and tiles that do not fit in shared memory.
+// grid read through L1/L2, takes the FP64 form and 3D windows wider than 16 taps.
 #include <math.h>
 
 #include "kernels_grad_tile.cuh"
@@ -65,8 +65,11 @@ static cudaError_t launch_grad_tile(const Plan& p, const void* g, const void* gr
 
 cudaError_t launch_interp_grad(const Plan& p, const void* g, const void* grad_f, double* grad_x, cudaStream_t st) {
   if (p.M == 0) return cudaSuccess;
-  // the shared-tile kernels' shared memory covers the tile and more than the exponential's table
-  if (p.prec == kF32 && p.tl.slab >= p.tl.E[0]) return launch_grad_tile(p, g, grad_f, grad_x, st);
+  // FP32 on staged tiles, in 3D up to 16 taps: above, the 6 W taps of a thread live in local memory
+  // (3D n = 128^3, 5e4 nodes, tile / thread per node: W = 16 0.92 / 1.07 ms, W = 18 3.5 / 1.5 ms,
+  // W = 24 37 / 3.2 ms; 2D n = 512^2, 1e5 nodes, W = 26 0.14 / 0.46 ms).  The shared-tile kernels'
+  // shared memory covers the tile and more than the exponential's table.
+  if (p.prec == kF32 && (p.geo.d < 3 || p.geo.W <= 16)) return launch_grad_tile(p, g, grad_f, grad_x, st);
   int64_t b = (p.M + 127) / 128;
   if (b > (int64_t)p.num_sms * 16) b = (int64_t)p.num_sms * 16;
   if (p.prec == kF64)
