@@ -34,7 +34,7 @@ namespace cg {
 
 constexpr int kNdftChunk = 256;
 constexpr int kNdftPairs = 32;   // pairs per block of the last dimension, at most
-constexpr int kNdftRowsF = 8;    // forward: rows per thread
+constexpr int kNdftRowsF = 8;    // forward: rows per thread, where there are more than two
 constexpr int kNdftRowsA = 32;   // adjoint: rows per CTA (4 per warp)
 constexpr int kNdftNodesA = 32;  // adjoint: nodes per stage
 
@@ -47,6 +47,7 @@ struct NdftRows {
   int64_t slow;    // combinations of the others
   int64_t groups;  // groups of consecutive rows along the fastest index
   int64_t per;     // rows per group
+  int xs;          // doubles from a node's coordinates to the next one's
 };
 
 __device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 acc) {
@@ -132,7 +133,7 @@ __device__ __noinline__ double2 ndft_node(const Geom& geo, const double2* __rest
 
 // coefficient i of an instance term by term
 template <int D>
-__device__ __noinline__ double2 ndft_coef(const Geom& geo, const double* __restrict__ x, const double2* __restrict__ f,
+__device__ __noinline__ double2 ndft_coef(const Geom& geo, const double* __restrict__ x, int xs, const double2* __restrict__ f,
                                           int64_t j0, int64_t j1, int64_t i) {
   double k[D];
 #pragma unroll
@@ -144,7 +145,7 @@ __device__ __noinline__ double2 ndft_coef(const Geom& geo, const double* __restr
   for (int64_t j = j0; j < j1; ++j) {
     double t = 0.0;
 #pragma unroll
-    for (int s = 0; s < D; ++s) t += turn(k[s], x[j * D + s]);
+    for (int s = 0; s < D; ++s) t += turn(k[s], x[j * xs + s]);
     acc = cfma(f[j], cis2pi(t), acc);
   }
   return acc;
@@ -155,7 +156,7 @@ __device__ __noinline__ double2 ndft_coef(const Geom& geo, const double* __restr
 template <int D, bool ADJ>
 __global__ void __launch_bounds__(256) k_ndft_add(const double* __restrict__ x, const double2* __restrict__ in,
                                                   const double2* __restrict__ part, double2* __restrict__ out, Geom geo,
-                                                  const int32_t* __restrict__ inst_off, int64_t n, int splits) {
+                                                  const int32_t* __restrict__ inst_off, int64_t n, int splits, int xs) {
   __shared__ double2 sum[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int64_t e0 = blockIdx.x * (int64_t)32; e0 < n; e0 += (int64_t)gridDim.x * 32) {
@@ -180,11 +181,11 @@ __global__ void __launch_bounds__(256) k_ndft_add(const double* __restrict__ x, 
       if (!finite2(v)) {
         if (ADJ) {
           const int64_t inst = e / geo.Ntot;
-          v = ndft_coef<D>(geo, x, in, inst_off[inst], inst_off[inst + 1], e - inst * geo.Ntot);
+          v = ndft_coef<D>(geo, x, xs, in, inst_off[inst], inst_off[inst + 1], e - inst * geo.Ntot);
         } else {
           int inst = 0;
           while (inst + 1 < geo.batch && inst_off[inst + 1] <= e) ++inst;
-          v = ndft_node<D>(geo, in + inst * geo.Ntot, x + e * D);
+          v = ndft_node<D>(geo, in + inst * geo.Ntot, x + e * xs);
         }
       }
       out[e] = v;
@@ -194,12 +195,11 @@ __global__ void __launch_bounds__(256) k_ndft_add(const double* __restrict__ x, 
 }
 
 // SPLIT: partial sums of split blockIdx.z to part [split][total], total nodes of all instances
-template <int D, bool SPLIT>
+template <int D, int R, bool SPLIT>
 __global__ void __launch_bounds__(128) k_ndft_forward(const double* __restrict__ x, const double2* __restrict__ fhat,
                                                       double2* __restrict__ f, Geom geo,
                                                       const int32_t* __restrict__ inst_off, NdftRows nr,
                                                       double2* __restrict__ part, int64_t total) {
-  constexpr int R = kNdftRowsF;
   __shared__ double2 sd[kNdftPairs][R][2];  // a+ + a-, -i (a+ - a-)
   const int inst = blockIdx.y;
   const int64_t j0 = inst_off[inst], j1 = inst_off[inst + 1];
@@ -214,10 +214,10 @@ __global__ void __launch_bounds__(128) k_ndft_forward(const double* __restrict__
     const bool on = j < j1;
     double xj[D];
 #pragma unroll
-    for (int t = 0; t < D; ++t) xj[t] = on ? x[j * D + t] : 0.0;
+    for (int t = 0; t < D; ++t) xj[t] = on ? x[j * nr.xs + t] : 0.0;
     const double xl = xj[D - 1];
     const double2 first = cis2pi(0.5 * xl), step = cis2pi(xl - rint(xl));
-    const double2 rstep = cis2pi(-(D == 1 ? turn((double)nr.B, xl) : xj[D > 1 ? D - 2 : 0]));
+    const double2 rstep = R > 1 ? cis2pi(-(D == 1 ? turn((double)nr.B, xl) : xj[D > 1 ? D - 2 : 0])) : first;
     double2 acc = make_double2(0.0, 0.0);
     for (int64_t g = g0; g < g1; ++g) {
       const NdftGroup<D> q = ndft_group<D>(geo, nr, g);
@@ -252,12 +252,12 @@ __global__ void __launch_bounds__(128) k_ndft_forward(const double* __restrict__
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         acc = cfma(s[r], rp, acc);
-        rp = cmul(rp, rstep);
+        if (R > 1) rp = cmul(rp, rstep);
       }
     }
     if (on) {
       if (SPLIT) part[blockIdx.z * total + j] = acc;
-      else f[j] = finite2(acc) ? acc : ndft_node<D>(geo, fh, x + j * D);
+      else f[j] = finite2(acc) ? acc : ndft_node<D>(geo, fh, x + j * nr.xs);
     }
   }
 }
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(256) k_ndft_adjoint(const double* __restrict__
       const int lo = (warp & 1) * SEG;
       double xj[D];
 #pragma unroll
-      for (int t = 0; t < D; ++t) xj[t] = x[(c0 + lane) * D + t];
+      for (int t = 0; t < D; ++t) xj[t] = x[(c0 + lane) * nr.xs + t];
       const double xl = xj[D - 1];
       if (warp < 2) {
         if (lo < half) {
@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(256) k_ndft_adjoint(const double* __restrict__
     const double2 vp = make_double2(A[r].x - Bv[r].y, A[r].y + Bv[r].x), vm = make_double2(A[r].x + Bv[r].y, A[r].y - Bv[r].x);
     auto put = [&](int64_t c, double2 v) {
       if (c >= NL) return;
-      out[row + c] = SPLIT || finite2(v) ? v : ndft_coef<D>(geo, x, f, j0, j1, row + c);
+      out[row + c] = SPLIT || finite2(v) ? v : ndft_coef<D>(geo, x, nr.xs, f, j0, j1, row + c);
     };
     put(cp, vp);
     put(cm, vm);
@@ -407,7 +407,7 @@ static int ndft_at_splits(const Plan& p, int64_t blocks, int64_t inner) {
 }
 
 // Blocks of the last dimension as equal as they come, of at most 2 kNdftPairs coefficients.
-static NdftRows ndft_rows(const Geom& geo, int per) {
+static NdftRows ndft_rows(const Geom& geo, int per, int xs) {
   NdftRows nr;
   const int64_t NL = geo.N[geo.d - 1];
   nr.nblk = (NL + 2 * kNdftPairs - 1) / (2 * kNdftPairs);
@@ -417,6 +417,7 @@ static NdftRows ndft_rows(const Geom& geo, int per) {
   nr.fast = geo.d == 1 ? nr.nblk : geo.N[geo.d - 2];
   nr.slow = geo.d == 1 ? 1 : nr.nblk * (geo.d == 3 ? geo.N[0] : 1);
   nr.per = per;
+  nr.xs = xs;
   nr.groups = (nr.fast + per - 1) / per;
   return nr;
 }
@@ -429,15 +430,25 @@ static int64_t max_nodes(const Plan& p) {
 
 // Launch of one direction: CTAs along nodes (forward) or row groups (adjoint), splits, results.
 struct NdftLaunch {
+  Geom geo;
   NdftRows nr;
   int threads;
   int64_t bx, splits, results;
 };
 
+// The geometry without trailing dimensions of one coefficient (frequency zero), which would leave
+// a block with one coefficient: N = 20000 x 1, M = 300 adjoint 1.68 ms, 0.06 as 1D.
+static Geom ndft_geom(Geom g) {
+  while (g.d > 1 && g.N[g.d - 1] == 1) --g.d;
+  return g;
+}
+
 static NdftLaunch ndft_launch_forward(const Plan& p) {
   NdftLaunch l;
   const int64_t maxM = max_nodes(p), want = (int64_t)p.num_sms * 6;
-  l.nr = ndft_rows(p.geo, kNdftRowsF);
+  l.geo = ndft_geom(p.geo);
+  l.nr = ndft_rows(l.geo, kNdftRowsF, p.geo.d);
+  if (l.nr.fast <= 2) l.nr = ndft_rows(l.geo, 1, p.geo.d);  // M = 1e5, N = 4: 66 us with 8 rows per thread, 38 with one; N = 64: 259, 83
   const int64_t ng = l.nr.slow * l.nr.groups;
   // one warp per CTA until there are enough CTAs to spread evenly over the SMs
   l.threads = (maxM + 127) / 128 * p.geo.batch * ng >= want ? 128 : 32;
@@ -453,7 +464,8 @@ static NdftLaunch ndft_launch_forward(const Plan& p) {
 static NdftLaunch ndft_launch_adjoint(const Plan& p) {
   NdftLaunch l;
   const int64_t maxM = max_nodes(p);
-  l.nr = ndft_rows(p.geo, kNdftRowsA);
+  l.geo = ndft_geom(p.geo);
+  l.nr = ndft_rows(l.geo, kNdftRowsA, p.geo.d);
   l.threads = 256;
   l.bx = l.nr.slow * l.nr.groups;
   // nodes split so that two CTAs run per SM, at least four nodes each
@@ -494,14 +506,19 @@ void ndft_release(Plan& p) {
 }
 
 template <bool ADJ>
-static cudaError_t add_partial_sums(const Plan& p, const double* x, const void* in, void* out, int64_t n, int splits,
+static cudaError_t add_partial_sums(const Plan& p, const NdftLaunch& l, const double* x, const void* in, void* out, int splits,
                                     cudaStream_t st) {
-  int64_t blocks = (n + 31) / 32;
+  int64_t blocks = (l.results + 31) / 32;
   if (blocks > (int64_t)p.num_sms * 8) blocks = (int64_t)p.num_sms * 8;
-  auto kern = p.geo.d == 1 ? k_ndft_add<1, ADJ> : (p.geo.d == 2 ? k_ndft_add<2, ADJ> : k_ndft_add<3, ADJ>);
-  kern<<<(unsigned)blocks, 256, 0, st>>>(x, (const double2*)in, (const double2*)p.nd_part, (double2*)out, p.geo, p.bins.inst_off,
-                                         n, splits);
+  auto kern = l.geo.d == 1 ? k_ndft_add<1, ADJ> : (l.geo.d == 2 ? k_ndft_add<2, ADJ> : k_ndft_add<3, ADJ>);
+  kern<<<(unsigned)blocks, 256, 0, st>>>(x, (const double2*)in, (const double2*)p.nd_part, (double2*)out, l.geo, p.bins.inst_off,
+                                         l.results, splits, l.nr.xs);
   return cudaGetLastError();
+}
+
+template <int R, bool SPLIT>
+static auto ndft_forward_kernel(int d) {
+  return d == 1 ? k_ndft_forward<1, R, SPLIT> : (d == 2 ? k_ndft_forward<2, R, SPLIT> : k_ndft_forward<3, R, SPLIT>);
 }
 
 cudaError_t launch_ndft_forward(Plan& p, const double* x, const void* fhat, void* f, cudaStream_t st) {
@@ -509,10 +526,10 @@ cudaError_t launch_ndft_forward(Plan& p, const double* x, const void* fhat, void
   const NdftLaunch l = ndft_launch_forward(p);
   const int64_t splits = ndft_splits(p, l, st);
   const dim3 grid((unsigned)l.bx, (unsigned)p.geo.batch, (unsigned)splits);
-  auto kern = splits > 1 ? (p.geo.d == 1 ? k_ndft_forward<1, true> : (p.geo.d == 2 ? k_ndft_forward<2, true> : k_ndft_forward<3, true>))
-                         : (p.geo.d == 1 ? k_ndft_forward<1, false> : (p.geo.d == 2 ? k_ndft_forward<2, false> : k_ndft_forward<3, false>));
-  kern<<<grid, l.threads, 0, st>>>(x, (const double2*)fhat, (double2*)f, p.geo, p.bins.inst_off, l.nr, (double2*)p.nd_part, p.M);
-  if (splits > 1) return add_partial_sums<false>(p, x, fhat, f, l.results, (int)splits, st);
+  auto kern = splits > 1 ? (l.nr.per == 1 ? ndft_forward_kernel<1, true>(l.geo.d) : ndft_forward_kernel<kNdftRowsF, true>(l.geo.d))
+                         : (l.nr.per == 1 ? ndft_forward_kernel<1, false>(l.geo.d) : ndft_forward_kernel<kNdftRowsF, false>(l.geo.d));
+  kern<<<grid, l.threads, 0, st>>>(x, (const double2*)fhat, (double2*)f, l.geo, p.bins.inst_off, l.nr, (double2*)p.nd_part, p.M);
+  if (splits > 1) return add_partial_sums<false>(p, l, x, fhat, f, (int)splits, st);
   return cudaGetLastError();
 }
 
@@ -534,10 +551,10 @@ cudaError_t launch_ndft_adjoint(Plan& p, const double* x, const void* f, void* f
   const NdftLaunch l = ndft_launch_adjoint(p);
   const int64_t splits = ndft_splits(p, l, st);
   const dim3 grid((unsigned)l.bx, (unsigned)p.geo.batch, (unsigned)splits);
-  auto kern = splits > 1 ? (p.geo.d == 1 ? k_ndft_adjoint<1, true> : (p.geo.d == 2 ? k_ndft_adjoint<2, true> : k_ndft_adjoint<3, true>))
-                         : (p.geo.d == 1 ? k_ndft_adjoint<1, false> : (p.geo.d == 2 ? k_ndft_adjoint<2, false> : k_ndft_adjoint<3, false>));
-  kern<<<grid, l.threads, 0, st>>>(x, (const double2*)f, (double2*)fhat, p.geo, p.bins.inst_off, l.nr, (double2*)p.nd_part);
-  if (splits > 1) return add_partial_sums<true>(p, x, f, fhat, l.results, (int)splits, st);
+  auto kern = splits > 1 ? (l.geo.d == 1 ? k_ndft_adjoint<1, true> : (l.geo.d == 2 ? k_ndft_adjoint<2, true> : k_ndft_adjoint<3, true>))
+                         : (l.geo.d == 1 ? k_ndft_adjoint<1, false> : (l.geo.d == 2 ? k_ndft_adjoint<2, false> : k_ndft_adjoint<3, false>));
+  kern<<<grid, l.threads, 0, st>>>(x, (const double2*)f, (double2*)fhat, l.geo, p.bins.inst_off, l.nr, (double2*)p.nd_part);
+  if (splits > 1) return add_partial_sums<true>(p, l, x, f, fhat, (int)splits, st);
   return cudaGetLastError();
 }
 

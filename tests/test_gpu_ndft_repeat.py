@@ -74,3 +74,38 @@ def test_sums_near_the_largest_number(N):
     assert ok.any() and torch.isfinite(torch.view_as_real(got[ok])).all()
     assert ((got[ok] * 1e-308 - ref[ok]).abs() < 1e-14).all()
     p.close()
+
+
+@pytest.mark.parametrize("N", [[30, 1], [9, 7, 1], [40, 1, 1], [1, 1], [1, 33, 1]])
+def test_trailing_dimensions_of_one_coefficient(N):
+    """Frequency zero only; the nodes keep their coordinates there (phases of k x rounded: 1e-12)."""
+    p, x, fh, f = _case(N, 250, 3)
+    xh = x.cpu().numpy()
+    assert O.rel_l2(O.ndft_forward(xh, fh.cpu().numpy(), N), p.ndft_forward(fh).cpu().numpy()) < 1e-12
+    got = p.ndft_adjoint(f).cpu().numpy()
+    assert O.rel_l2(O.ndft_adjoint(xh, f.cpu().numpy(), N).reshape(got.shape), got) < 1e-12
+    f[3] = float("inf")
+    assert torch.isinf(torch.view_as_real(p.ndft_adjoint(f)).reshape(-1)[::2]).any()
+    p.close()
+
+
+@pytest.mark.parametrize("N,like,M,adjoint,factor", [([64], [8, 8], 100000, False, 1.5), ([20000, 1], [20000], 300, True, 3.0),
+                                                     ([300, 1, 1], [300], 5000, True, 3.0)])
+def test_few_rows_take_no_longer(N, like, M, adjoint, factor):
+    """As long as another shape of as many terms (an eighth of the work was used at N = 64, a
+    thirtieth with a last dimension of one)."""
+    took = []
+    for shape in (N, like):
+        p, x, fh, f = _case(shape, M)
+        times = []
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            a.record()
+            p.ndft_adjoint(f) if adjoint else p.ndft_forward(fh)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        took.append(min(times))
+        p.close()
+    assert took[0] < factor * took[1], took
