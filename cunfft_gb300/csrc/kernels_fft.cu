@@ -434,7 +434,7 @@ void fft_fix_release(Plan& p) {
 }
 
 // Tables of the FP64 form's FFT, where it covers the grid: power-of-two sizes of 16 to 4096
-// points (1D: to 2^24, with a second buffer of at most 1 GB).  The plan keeps the library's
+// points (1D: to 2^24, with a second buffer of at most 1 GB).  The plan takes the library's
 // FFT for everything else, and where the memory cannot be had.
 void fft_fix_prepare(Plan& p) {
   const Geom& g = p.geo;

@@ -461,18 +461,16 @@ int plan_init(Plan* p, int d, const int64_t* N, const int64_t* n, int m, int pre
     CG_TRY(check_cuda(p, plan_malloc(&p->g, elem_bytes(p) * g.ntot * batch), "cudaMalloc grid"));
     p->own_g = true;
   }
-  // batched in-place FFT over the instances' grids
-  {
-    int nn[kMaxDim];
-    for (int t = 0; t < d; ++t) {
-      if (g.n[t] > 0x7fffffff) return set_status(p, CUNFFT_X_UNSUPPORTED, "FFT length too large");
-      nn[t] = (int)g.n[t];
-    }
+  // batched in-place FFT over the instances' grids: the FP64 form's own, or a library plan
+  for (int t = 0; t < d; ++t)
+    if (g.n[t] > 0x7fffffff) return set_status(p, CUNFFT_X_UNSUPPORTED, "FFT length too large");
+  fft_fix_prepare(*p);
+  if (!p->fx_on) {
     cufftHandle h;
     CG_TRY(check_cufft(p, cufftCreate(&h), "cufftCreate"));
     size_t ws = 0;
     long long nll[kMaxDim];
-    for (int t = 0; t < d; ++t) nll[t] = nn[t];
+    for (int t = 0; t < d; ++t) nll[t] = g.n[t];
     cufftResult r = plan_fft_fault() ? CUFFT_INTERNAL_ERROR
                                      : cufftMakePlanMany64(h, d, nll, nullptr, 1, g.ntot, nullptr, 1, g.ntot,
                                                            prec == kF64 ? CUFFT_Z2Z : CUFFT_C2C, batch, &ws);
@@ -482,7 +480,6 @@ int plan_init(Plan* p, int d, const int64_t* N, const int64_t* n, int m, int pre
     }
     p->fft = h;
     p->own_fft = true;
-    fft_fix_prepare(*p);
   }
   // per-instance node offsets, status flag, work counters
   CG_TRY(check_cuda(p, plan_malloc(&p->bins.inst_off, sizeof(int32_t) * (batch + 1)), "cudaMalloc"));

@@ -28,10 +28,10 @@ struct Plan {
   int device = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
-  cufftHandle fft = 0;         // batched plan used for both directions
+  cufftHandle fft = 0;         // batched plan used for both directions (0 with fx_on)
   bool own_fft = false;
-  // FP64 form: twiddle tables and 1D scratch of the fixed-point FFT (kernels_fft.cu); off:
-  // the library's FFT
+  // FP64 form: twiddle tables and 1D scratch (at most 1 GB) of the fixed-point FFT
+  // (kernels_fft.cu); off: the library's FFT
   int4* fx_tab = nullptr;
   void* fx_tmp = nullptr;
   int64_t fx_off[4] = {0, 0, 0, 0};

@@ -246,8 +246,11 @@ int cunfft_x_get_interp_kernel(const cunfft_x_plan *plan, int *kind);
 /** Per-stage device times of the last forward/adjoint call, in seconds
  *  (binning, roll-off, FFT, gridding), by stage whatever the direction: after an
  *  adjoint, t_conv is the spreading and t_roc the crop (the reference fills
- *  CUNFFTTimes the same way, src/cunfft.cu:209-224).  Blocks until the plan stream
- *  is idle. */
+ *  CUNFFTTimes the same way, src/cunfft.cu:209-224).  FP64 plans on power-of-two grids
+ *  (16 to 4096 points per dimension, 1D to 2^24) apply the roll-off of a forward in the
+ *  FFT's first pass: its time counts as the FFT's, t_roc is near zero (so is time_ROC of
+ *  the reference's interface, whose fft_forward and fft_backward handles such grids do
+ *  not use).  Blocks until the plan stream is idle. */
 int cunfft_x_stage_times(cunfft_x_plan *plan, double *t_bin, double *t_roc, double *t_fft, double *t_conv);
 
 /** Forward transform between host buffers, with the copies on the plan's two copy
