@@ -26,8 +26,9 @@ class NFFT:
     # plans with a private stream per device: with one alone nothing has to be held (making another
     # waits for the work of those before it)
     _private_plans = collections.Counter()
-    # tensors held before an event is spent on them (one is a gap of some 15 us in the stream)
-    _HELD_BYTES = 256 << 20
+    # tensors and calls held before an event is spent on them (one is a gap of some 15 us in the
+    # stream; more calls only make the allocator's pool grow)
+    _HELD_BYTES, _HELD_CALLS = 256 << 20, 32
 
     def __init__(self, N, n=None, m=6, precision="f64", batch=1, device=None, stream=None, window="gaussian"):
         self._host_refs = []  # host tensors in flight in host-buffer transforms
@@ -111,7 +112,7 @@ class NFFT:
         self.M_inst = M_inst
         self.M = M
         call = 2 * (self.cdtype.itemsize * (self.batch * self.N_total + M) + 8 * self.d * M)
-        self._open_calls = max(1, NFFT._HELD_BYTES // max(1, call))
+        self._open_calls = min(NFFT._HELD_CALLS, max(1, NFFT._HELD_BYTES // max(1, call)))
         return self
 
     # ------------------------------------------------------------ transforms
@@ -132,8 +133,9 @@ class NFFT:
         until a later batch finds the work before it done, synchronize() or close()."""
         if self._private is None or NFFT._private_plans[self._index] < 2:
             return
-        self._open.append([t.detach() if t.requires_grad else t for t in tensors])  # without an autograd graph
-        if len(self._open) < self._open_calls:
+        for t in tensors:
+            self._open.append(t.detach() if t.requires_grad else t)  # without an autograd graph
+        if len(self._open) < 2 * self._open_calls:
             return
         done = torch.cuda.Event()
         done.record(self._private)
@@ -149,10 +151,12 @@ class NFFT:
             return
         if a.requires_grad or out.requires_grad:
             a, out = a.detach(), out.detach()
-        before = self._live.get(what)
-        self._live[what] = (a, out)
-        if before is not None and (before[0] is not a or before[1] is not out):  # a loop's fixed buffers stay
-            self._keep(*before)
+        before, self._live[what] = self._live.get(what), (a, out)
+        if before is not None:  # a loop's fixed buffers stay
+            if before[1] is not out:
+                self._keep(before[1])
+            if before[0] is not a:
+                self._keep(before[0])
 
     def _release(self):
         self._pending.clear()
@@ -303,6 +307,7 @@ class NFFT:
         nat.check(self._lib.cunfft_x_get_window(self._h, ctypes.byref(k)))
         return {v: n for n, v in self.WINDOWS.items()}[k.value]
 
+    # ("global" is refused: no plan runs such a kernel)
     SPREAD_KERNELS = {"auto": 0, "shared": 1, "register": 2, "global": 3, "tensor": 4}
 
     def set_spread_kernel(self, kind="auto"):
@@ -310,7 +315,7 @@ class NFFT:
         nat.check(self._lib.cunfft_x_set_spread_kernel(self._h, self.SPREAD_KERNELS[kind]), self._h)
 
     def spread_kernel(self):
-        """Spreading kernel in use: "shared", "register", "tensor" or "global"."""
+        """Spreading kernel in use: "shared", "register" or "tensor"."""
         k = ctypes.c_int()
         nat.check(self._lib.cunfft_x_get_spread_kernel(self._h, ctypes.byref(k)))
         return {v: n for n, v in self.SPREAD_KERNELS.items()}[k.value]
@@ -322,7 +327,7 @@ class NFFT:
         nat.check(self._lib.cunfft_x_set_interp_kernel(self._h, self.INTERP_KERNELS[kind]), self._h)
 
     def interp_kernel(self):
-        """Interpolation kernel in use: "shared", "tensor" or "global"."""
+        """Interpolation kernel in use: "shared" or "tensor"."""
         k = ctypes.c_int()
         nat.check(self._lib.cunfft_x_get_interp_kernel(self._h, ctypes.byref(k)))
         return {v: n for n, v in self.INTERP_KERNELS.items()}[k.value]
