@@ -29,10 +29,13 @@
 //    node), as are the samples of an item with a fraction that is not finite.
 //
 // Measured against the FP64-pipe kernels before: 3D n = 128^3, M = 2^18, m = 6 interpolation
-// 4.18 -> 0.94 ms, spreading 5.75 -> 1.61 ms; m = 12 (global-memory kernels before)
-// 68.8 -> 5.9 and 43.2 -> 9.8 ms; 2D n = 1024^2, M = 2^18, m = 6 0.80 -> 0.16 and
-// 1.00 -> 0.28 ms.  Relative l2 error against 64-bit sums with exact taps: 4e-16 to 1.1e-15
-// for whole m = 6 transforms (4e-15 to 1.5e-14 before, from the recurrence taps).
+// 4.18 -> 0.96 ms, spreading 5.75 -> 1.57 ms; m = 12 (global-memory kernels before)
+// 68.8 -> 6.0 and 43.2 -> 9.9 ms; 2D n = 1024^2, M = 2^18, m = 6 0.80 -> 0.16 and
+// 1.00 -> 0.28 ms.  Relative l2 error of whole transforms against 64-bit sums with exact taps
+// (before, from the recurrence taps): m = 6 3e-16 to 1.2e-15 (2e-15 to 1.5e-14); 3D, m = 12,
+// where the grid's values cancel 24-fold in the window's sum and the roll-off raises the
+// spreading's rounding as much, forward 4e-16 to 9.8e-15 (9e-15 to 4.3e-14), adjoint 3e-16 to
+// 6.1e-14 (1.5e-14 to 7.0e-14).
 #pragma once
 
 #include "fixmath.h"

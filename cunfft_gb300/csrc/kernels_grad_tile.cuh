@@ -6,8 +6,9 @@
 // wavefronts instead of up to 32 cache lines, and the taps w and const y w are formed in
 // integers (fixmath.h) and rounded to FP32 once, as FP64 taps would be, instead of FP64
 // exponentials.
-// Bound: shared-memory wavefronts of scattered reads (about seven for a warp's 32 windows).
-// 2D, m = 6, M = 2^18: 93 us; gathers from global memory and FP64 taps before: 400 us.
+// Bound: shared-memory wavefronts of scattered reads (about seven for a warp's 32 windows), the
+// FP64 pipe (coordinates) and the integer multiply-adds (taps) close to one another.
+// 2D, m = 6, M = 2^18: 92 us; gathers from global memory and FP64 taps before: 400 us.
 #pragma once
 
 #include "kernels_fix.cuh"

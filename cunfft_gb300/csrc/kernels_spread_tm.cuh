@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) k_spread_tm(const float2* __res
   bool healthy = true;
 
   // Every role walks the same items (tm_next_item); batch gb (counted across the CTA's
-  // items) uses stage gb % 4 in its cycle gb / 4 and record / table buffers gb & 1.
+  // items) uses stage gb % kTmStages in its cycle gb / kTmStages and table buffers gb & 1.
   // A role whose bounded wait gives up raises abort_flag and leaves its loop; the
   // builders leave together after their barrier, the others at their next wait, so a
   // broken hand-off ends the kernel after a few bounded waits instead of one per batch.
