@@ -65,8 +65,10 @@ def test_no_block_in_use_is_another_plans_output(name):
 
 def test_held_tensors_are_released():
     """Calls on a plan whose work is done do not pile up memory, and none stays with synchronize()."""
+    import gc
     (p, other), x, fh, f = _plans()
     torch.cuda.synchronize()
+    gc.collect()  # other tests' tensors
     before = torch.cuda.memory_allocated()
     one = p.forward(fh).nbytes + p.node_gradient(fh, f).nbytes + p.interp(torch.ones(p.n, dtype=torch.complex128, device="cuda:0")).nbytes
     for _ in range(60):
