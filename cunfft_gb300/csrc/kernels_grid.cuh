@@ -33,7 +33,11 @@
 //    load / FMA / store; for d = 1 each warp accumulates into a private copy of
 //    the tile.  Batches are double-buffered (one barrier per batch).  The tile is
 //    then added to the global grid with vector atomics, so neighbouring items'
-//    halos combine.
+//    halos combine.  In 1D and 2D eight CTAs form a cluster, take neighbouring items
+//    and add the tiles of one grid tile over their shared memory first: shorter items
+//    for the SMs (eight times as many partial sums on a cell, added in FP32) had raised
+//    the error of dense grids of few tiles (N = 173, m = 4, M = 1e5: 2.1e-7 with items of
+//    2048 nodes, 3.0e-7 with 256, 2.1e-7 with 256 in clusters; adjoint 113, 54, 58 us).
 //  * Wide windows in 3D: above 16 taps a warp's lanes take consecutive cells of a plane's
 //    W x W window (interpolation; one row of W taps per pass left 32 - W lanes idle), and
 //    above 24 taps, where the padded tile of a single plane of window starts does not fit
@@ -263,14 +267,15 @@ __device__ __forceinline__ void load_tile(C* tile, const C* __restrict__ gi, con
 
 // Add the tile into the global grid.  FP32 pairs (even offset on a 16-byte aligned grid
 // whose last size is even, so 16-byte aligned and never split by the wrap) go as one
-// float4 atomic.
+// float4 atomic.  Of `parts` > 1 parts (d <= 2), this call adds part `part`: rows part,
+// part + parts, ... (d = 1: pairs of cells).
 template <int D, int W, typename C>
 __device__ __forceinline__ void flush_tile(const C* tile, C* __restrict__ gi, const Geom& geo, const Tiling& tl,
-                                           const TileOrigin& o, int p_lo, int p_n) {
+                                           const TileOrigin& o, int p_lo, int p_n, int part = 0, int parts = 1) {
   constexpr int S = TileShape<D, W, C>::S, PS = TileShape<D, W, C>::PS;
   const int E_last = tl.E[D - 1];
   const int64_t n_last = geo.n[D - 1], a_last = o.a[D - 1];
-  const int rows = D == 3 ? p_n * tl.E[1] : tile_rows<D>(tl);
+  const int rows = D == 3 ? p_n * tl.E[1] : (D == 2 ? (tl.E[0] - part + parts - 1) / parts : 1);
   constexpr bool kF32 = sizeof(C) == 8;
   const int tid = threadIdx.x, nt = blockDim.x;
   const bool pairs_ok = kF32 && (n_last & 1) == 0 && (tl.T[D - 1] & 1) == 0 &&  // even tile origin and row length
@@ -279,8 +284,9 @@ __device__ __forceinline__ void flush_tile(const C* tile, C* __restrict__ gi, co
   const int total = rows * per_row;
   for (int e = tid; e < total; e += nt) {
     const int row = e / per_row, k = e - row * per_row;
+    if (D == 1 && parts > 1 && (pairs_ok ? k : k >> 1) % parts != part) continue;
     int p0, p1;
-    row_coords<D>(tl, row, &p0, &p1);
+    row_coords<D>(tl, D == 2 ? part + row * parts : row, &p0, &p1);
     const C* src = tile + (D == 3 ? p0 * PS + p1 * S : (D == 2 ? p0 * S : 0));
     const int64_t gb = row_gbase<D>(geo, o, p0 + p_lo, p1);
     if (pairs_ok) {
@@ -309,6 +315,32 @@ __device__ __forceinline__ bool next_item(const Bins& bins, int slot, int4* cur)
   }
   __syncthreads();
   return cur->x >= 0;
+}
+
+// CTAs per cluster of the FP32 spreading in 1D and 2D: they take neighbouring items, and add the
+// tiles of one grid tile before they go to the grid.
+template <int D, typename T>
+__host__ __device__ constexpr int spread_cluster() {
+  return D < 3 && sizeof(T) == 4 ? 8 : 1;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive;\n\tbarrier.cluster.wait;" ::: "memory");
+}
+// what CTA `rank` of the cluster has at this CTA's address p
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, int rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float2 cluster_load(const float2* p, int rank) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(cluster_addr(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ int cluster_load(const int* p, int rank) {
+  int v;
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(cluster_addr(p, rank)) : "memory");
+  return v;
 }
 
 // Shared-memory bytes beyond the tile, per kernel kind (the host sizes launches with it).
@@ -561,8 +593,34 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 256 : 512) k_spread(const typ
   // this thread's staging role: (node, dim) for weights, node for records
   const int sq = threadIdx.x / D, st = threadIdx.x - sq * D;
 
-  while (next_item(bins, 1, &cur)) {
-    const int4 item = cur;
+  // CL > 1: the cluster's CTAs take CL neighbouring items at a time.  CTA 0 draws the next group
+  // while the present one runs; the barriers of a group publish it.
+  constexpr int CL = spread_cluster<D, T>();
+  const int rank = CL > 1 ? (int)(blockIdx.x % CL) : 0, num = CL > 1 ? *bins.num_items : 0;
+  __shared__ int s_next[2];
+  auto draw = [&](int slot) {
+    if (rank == 0 && threadIdx.x == 0) s_next[slot] = atomicAdd(&bins.work[1], CL);
+  };
+  if constexpr (CL > 1) {
+    draw(0);
+    cluster_sync();
+  }
+  for (int turn = 0;; turn ^= 1) {
+    int4 item;
+    int valid = 1;      // items of the group
+    bool same = false;  // of one tile
+    if constexpr (CL > 1) {
+      const int base = cluster_load(&s_next[turn], 0);
+      if (base >= num) break;
+      draw(turn ^ 1);
+      valid = min(CL, num - base);
+      const int t = bins.items[base + min(lane & (CL - 1), valid - 1)].x, t0 = __shfl_sync(0xffffffffu, t, 0);
+      same = valid > 1 && __all_sync(0xffffffffu, t == t0);
+      item = rank < valid ? bins.items[base + rank] : make_int4(t0, 0, 0, 0);
+    } else {
+      if (!next_item(bins, 1, &cur)) break;
+      item = cur;
+    }
     const TileOrigin o = decode_tile<D>(geo, tl, item.x);
     for (int p_lo = 0; p_lo < (SLAB ? tl.E[0] : 1); p_lo += SLAB ? tl.slab : 1) {
       const int p_n = SLAB ? min(tl.slab, tl.E[0] - p_lo) : tl.E[0];
@@ -682,10 +740,35 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 256 : 512) k_spread(const typ
         }
         __syncthreads();
       }
-      flush_tile<D, W, C>(tile, g + o.inst * geo.ntot, geo, tl, o, p_lo, p_n);
-      __syncthreads();
+      if constexpr (CL > 1) {
+        cluster_sync();
+        if (same) {  // this CTA's part of the sum over the cluster's tiles, in place
+          const int rows = D == 2 ? (tl.E[0] - rank + CL - 1) / CL : 1;
+          const int cols = D == 2 ? tl.E[1] : tl.E[0];
+          for (int e = threadIdx.x; e < rows * cols; e += blockDim.x) {
+            const int row = e / cols, c = e - row * cols;
+            if (D == 1 && (c >> 1) % CL != rank) continue;
+            C* const p = tile + (D == 2 ? (rank + row * CL) * S : 0) + c;
+            C v = cluster_load(p, 0);
+            for (int q = 1; q < valid; ++q) {
+              const C w = cluster_load(p, q);
+              v.x += w.x;
+              v.y += w.y;
+            }
+            *p = v;
+          }
+          __syncthreads();
+        }
+        if (same) flush_tile<D, W, C>(tile, g + o.inst * geo.ntot, geo, tl, o, p_lo, p_n, rank, CL);
+        else if (rank < valid) flush_tile<D, W, C>(tile, g + o.inst * geo.ntot, geo, tl, o, p_lo, p_n);
+        cluster_sync();  // every tile read before it is cleared
+      } else {
+        flush_tile<D, W, C>(tile, g + o.inst * geo.ntot, geo, tl, o, p_lo, p_n);
+        __syncthreads();
+      }
     }
   }
+  if constexpr (CL > 1) cluster_sync();  // CTA 0's last draw has been read
 }
 
 // One node through global memory: interpolation of the grid at the node (out[idx] written)
