@@ -74,7 +74,10 @@ typedef struct cunfft_x_plan cunfft_x_plan;
  *  last size (spreading) or one divisible by 8 (interpolation), other sizes run the
  *  shared-tile forms; the 2D tensor-core spreading takes any size.  1 <= m <= 15; precision CUNFFT_X_F64 or
  *  CUNFFT_X_F32; batch >= 1 instances; stream 0 creates a private stream
- *  (a cudaStream_t may be passed as void*). */
+ *  (a cudaStream_t may be passed as void*).  FP64 plans whose sizes are powers of two
+ *  (16 to 4096, 1D to 2^24) hold their own FFT's tables in place of a cuFFT plan; 1D
+ *  sizes above 4096 also a second grid, of at most 1 GB over the instances (larger plans,
+ *  or no memory for it: cuFFT). */
 int cunfft_x_plan_create(cunfft_x_plan **plan, int d, const int64_t *N, const int64_t *n, int m,
                          int precision, int batch, void *stream);
 
